@@ -120,11 +120,10 @@ int tb_block_multiply(double alpha, const double* a, const int64_t* adims, const
   std::unique_ptr<WorkList> wl(single_block_worklist(plan.lc, adims, bdims, cdims));
   auto st = static_cast<cudaStream_t>(stream);
   WorkList& w = *wl;
-  finalize_worklist(plan.lc, w);
-  if(mode == TB_MODE_FP64 || plan.lc.nar > 0 || plan.lc.nbr > 0) {
-    // A-only / B-only reduction steps are beta-chained on the FP64 tensor-core path.
-    launch_contract_fp64(plan, w, alpha, beta, is_assign, a, b, c, st);
-  }
+  // A-only / B-only reduction steps are beta-chained on the FP64 tensor-core path.
+  const bool fp64 = mode == TB_MODE_FP64 || plan.lc.nar > 0 || plan.lc.nbr > 0;
+  finalize_worklist(plan.lc, w, !fp64);
+  if(fp64) launch_block_fp64(plan.lc, w.groups[0], w.tasks[0], alpha, beta, is_assign, a, b, c, st);
   else {
     if(is_assign) launch_fill(c, [&] {
         int64_t n = 1;
@@ -134,6 +133,7 @@ int tb_block_multiply(double alpha, const double* a, const int64_t* adims, const
     run_contract(plan, w, alpha, a, b, c, st, nullptr);
   }
   TB_CUDA(cudaStreamSynchronize(st)); // the work list is released on return
+  check_wait_errors();
   TB_API_END
 }
 
@@ -349,6 +349,7 @@ int tb_ctx_synchronize(tb_ctx ctx) {
   TB_CUDA(cudaStreamSynchronize(ctx->p->stream));
   if(ctx->p->h2d) TB_CUDA(cudaStreamSynchronize(ctx->p->h2d));
   if(ctx->p->d2h) TB_CUDA(cudaStreamSynchronize(ctx->p->d2h));
+  check_wait_errors();
   TB_API_END
 }
 
@@ -1111,6 +1112,7 @@ int tb_sched_execute(tb_sched s, int hw, int profile) {
   TB_EXPECTS(hw >= 0 && hw <= 2, "hw must be 0 (DEFAULT), 1 (CPU) or 2 (GPU)");
   s->p->execute(profile != 0);
   TB_CUDA(cudaStreamSynchronize(s->p->ctx->stream));
+  check_wait_errors();
   TB_API_END
 }
 
@@ -1139,6 +1141,7 @@ int tb_sched_wait(tb_sched s) {
   auto pending = std::move(s->p->pending);
   s->p->pending.clear();
   for(const auto& wl: pending) check_int8_errors(*wl, c.stream);
+  check_wait_errors();
   TB_API_END
 }
 
@@ -1374,6 +1377,7 @@ int tb_graph_sync(tb_graph g) {
   TB_CUDA(cudaSetDevice(g->p->ctx->device));
   TB_CUDA(cudaStreamSynchronize(g->p->ctx->stream));
   for(const auto& wl: g->p->int8_lists) check_int8_errors(*wl, g->p->ctx->stream);
+  check_wait_errors();
   TB_API_END
 }
 

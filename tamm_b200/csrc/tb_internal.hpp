@@ -71,16 +71,26 @@ struct DevTask {
   int64_t a_off, b_off;
   int32_t adims[kMaxModes];
   int32_t bdims[kMaxModes];
+  int32_t pos, pad; // K chunks of the group's admitted tasks before this one, run or skipped
 };
-// One CTA's output tile: group, batch index, first row / column of the tile.
+constexpr int kChunkK = 32; // K elements per chunk of the FP64 kernel
+// One CTA's work in the FP64 kernel: an output tile (group, batch index, first row /
+// column) run whole (nparts = 1), or one segment of its K: `nchunks` chunks from chunk
+// `chunk0` of task `task0` on, the `part`th nonempty one of `nparts`, whose accumulators
+// go to slot ws + part of the workspace.  `tile` numbers the tiles of the launch; a whole
+// tile of nseg > 1 segments over `total` chunk positions closes a partial sum at each.
 struct DevItem {
   int32_t group, batch, m0, n0;
+  int32_t task0, chunk0, nchunks;
+  int32_t tile, part, nparts, ws;
+  int32_t total, nseg;
 };
 
 // Host mirror of a work list plus its device copies.
 struct WorkList {
   std::vector<DevGroup> groups;
   std::vector<DevTask>  tasks;
+  std::vector<int32_t>  group_chunks;      // K chunks of each group's admitted tasks, run or skipped
   double                flops = 0;         // admitted FP64 FLOPs (tasks that run + skipped tasks)
   double                flops_run = 0;     // FP64 FLOPs of the tasks in the list
   double                flops_skipped = 0; // admitted tasks left out: an exactly-zero block of a read-only operand
@@ -92,8 +102,12 @@ struct WorkList {
   // work list: contractions that run split-INT8 or BF16x3 never need them
   mutable std::vector<DevItem> items_fp64;
   mutable DevItem*             d_items     = nullptr;
+  mutable void *               d_group_recs = nullptr, *d_task_recs = nullptr; // (d_group_recs: the block of all three)
   mutable bool                 items_built = false;
-  mutable int                  items_bn    = 64; // output tile width of those items
+  mutable int                  items_shape = 64; // tile shape of those items, by its width
+  mutable int64_t              ntiles_fp64 = 0;  // output tiles
+  mutable int64_t              split_parts = 0;  // segments that run as items of their own
+  mutable bool                 multi_segment = false; // a tile of several segments runs whole
   ~WorkList();
 };
 
@@ -182,9 +196,17 @@ struct Plan {
   int64_t*      cache_used  = nullptr;
 };
 
+// Error word of the FP64 contraction's device-side waits on the current device, in host
+// memory mapped to the GPU, so that the host reads it without a copy once the launch has
+// finished; check_wait_errors() throws TB_ERR_TIMEOUT if a wait gave up since the last
+// check, and clears it.
+int*  wait_error_word();
+void  check_wait_errors();
 void forget_int8_layout(const WorkList* wl);
 // FP64 FLOPs of one task of a group (2 * |C block| * K, times the one-sided steps).
 double task_flops(const LabelClasses& lc, const DevGroup& g, const DevTask& t);
+// K chunks of one task, over all its one-sided reduction steps.
+int64_t task_chunks(const LabelClasses& lc, const DevTask& t);
 // Largest split-INT8 slice count the error target needs (3..8).
 int int8_slices_for(double err_target);
 
@@ -192,6 +214,9 @@ int int8_slices_for(double err_target);
 void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, double beta,
                           int is_assign, const double* A, const double* B, double* C,
                           cudaStream_t stream);
+// The same for one block triple, without a work list in device memory.
+void launch_block_fp64(const LabelClasses& lc, const DevGroup& g, const DevTask& t, double alpha, double beta,
+                       int is_assign, const double* A, const double* B, double* C, cudaStream_t stream);
 void contract_int8(Plan& plan, const WorkList& wl, double alpha, const double* A,
                    const double* B, double* C, cudaStream_t stream);
 void contract_bf16x3(Plan& plan, const WorkList& wl, double alpha, const double* A,

@@ -107,13 +107,13 @@ LabelClasses classify(const int* cl, int nc, const int* al, int na, const int* b
 
 WorkList::~WorkList() {
   forget_int8_layout(this);
-  if(d_groups || d_tasks || d_items) {
+  if(d_groups || d_tasks || d_group_recs) {
     int cur = -1;
     cudaGetDevice(&cur);
     if(device >= 0) cudaSetDevice(device);
     cudaFree(d_groups);
     cudaFree(d_tasks);
-    cudaFree(d_items);
+    cudaFree(d_group_recs);
     if(cur >= 0) cudaSetDevice(cur);
   }
 }
@@ -154,16 +154,32 @@ double task_flops(const LabelClasses& lc, const DevGroup& g, const DevTask& t) {
   return 2.0 * csz * k;
 }
 
+int64_t task_chunks(const LabelClasses& lc, const DevTask& t) {
+  int64_t k = 1, steps = 1;
+  for(int j = 0; j < lc.nk; j++) k *= t.adims[lc.k_a[j]];
+  for(int j = 0; j < lc.nar; j++) steps *= t.adims[lc.ar_a[j]];
+  for(int j = 0; j < lc.nbr; j++) steps *= t.bdims[lc.br_b[j]];
+  return steps * ((k + kChunkK - 1) / kChunkK);
+}
+
 void finalize_worklist(const LabelClasses& lc, WorkList& wl, bool upload) {
   wl.flops_run = 0;
+  const bool positions = wl.group_chunks.size() != wl.groups.size(); // not given: no task was skipped
+  if(positions) wl.group_chunks.assign(wl.groups.size(), 0);
   for(const auto& g: wl.groups) {
     TB_EXPECTS(g.task_begin >= 0 && g.task_end >= g.task_begin &&
                  g.task_end <= (int64_t) wl.tasks.size(),
                "group task range out of bounds");
+    int64_t chunks = 0;
     for(int t = g.task_begin; t < g.task_end; t++) {
       validate_task(lc, g, wl.tasks[t]);
       wl.flops_run += task_flops(lc, g, wl.tasks[t]);
+      if(!positions) continue;
+      wl.tasks[t].pos = (int32_t) chunks;
+      chunks += task_chunks(lc, wl.tasks[t]);
+      TB_EXPECTS(chunks < (1ll << 31), "contraction too long");
     }
+    if(positions) wl.group_chunks[&g - wl.groups.data()] = (int32_t) chunks;
   }
   wl.flops = wl.flops_run + wl.flops_skipped;
   if(!upload) return;

@@ -4,6 +4,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstring>
+#include <mutex>
 #include <numeric>
 #include <sstream>
 
@@ -89,10 +90,66 @@ void Arena::deallocate(void* p) {
   add_free(start, sz);
 }
 
+// Stream-ordered pool of a device for scratch without an arena.  Up to kPoolKeep bytes
+// stay with the pool between calls (the default pool hands all of it back at every
+// synchronisation, and mapping it again costs more than a small contraction).
+static cudaMemPool_t scratch_pool() {
+  constexpr uint64_t    kPoolKeep = uint64_t(128) << 20;
+  static cudaMemPool_t  pools[64] = {nullptr};
+  static std::once_flag once[64];
+  int                   dev = 0;
+  TB_CUDA(cudaGetDevice(&dev));
+  TB_EXPECTS(dev >= 0 && dev < 64, "device index out of range");
+  std::call_once(once[dev], [dev] {
+    cudaMemPoolProps props{};
+    props.allocType     = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id   = dev;
+    cudaMemPool_t pool  = nullptr;
+    TB_CUDA(cudaMemPoolCreate(&pool, &props)); // throws: the flag stays unset
+    uint64_t keep = kPoolKeep;
+    TB_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    pools[dev] = pool;
+  });
+  return pools[dev];
+}
+
+namespace {
+int*           g_wait_words = nullptr; // one 128-byte line per device
+std::once_flag g_wait_once;
+} // namespace
+
+int* wait_error_word() {
+  std::call_once(g_wait_once, [] {
+    void* p = nullptr;
+    TB_CUDA(cudaHostAlloc(&p, 64 * 128, cudaHostAllocMapped | cudaHostAllocPortable)); // throws: the flag stays unset
+    std::memset(p, 0, 64 * 128);
+    g_wait_words = static_cast<int*>(p);
+  });
+  int dev = 0;
+  TB_CUDA(cudaGetDevice(&dev));
+  TB_EXPECTS(dev >= 0 && dev < 64, "device index out of range");
+  void* d = nullptr;
+  TB_CUDA(cudaHostGetDevicePointer(&d, g_wait_words + 32 * dev, 0));
+  return static_cast<int*>(d);
+}
+
+void check_wait_errors() {
+  if(g_wait_words == nullptr) return;
+  int dev = 0;
+  TB_CUDA(cudaGetDevice(&dev));
+  if(dev < 0 || dev >= 64) return;
+  volatile int* w = g_wait_words + 32 * dev;
+  const int     h = *w;
+  if(h == 0) return;
+  *w = 0;
+  fail(TB_ERR_TIMEOUT, "FP64 contraction: a device-side wait gave up (code " + std::to_string(h) + ")");
+}
+
 void* Scratch::get(int64_t bytes) {
   if(arena) return arena->allocate(bytes);
   void* p = nullptr;
-  TB_CUDA(cudaMallocAsync(&p, (size_t) std::max<int64_t>(bytes, 1), stream));
+  TB_CUDA(cudaMallocFromPoolAsync(&p, (size_t) std::max<int64_t>(bytes, 1), scratch_pool(), stream));
   return p;
 }
 
@@ -554,7 +611,7 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
     g.task_begin = (int32_t) wl->tasks.size();
     std::fill(inner.begin(), inner.end(), 0);
     double  gskip  = 0; // FLOPs and count of this group's skipped tasks
-    int64_t gskipn = 0;
+    int64_t gskipn = 0, gchunks = 0;
     do {
       for(size_t i = 0; i < aid.size(); i++) {
         int64_t l = a_out[i] >= 0 ? itval[a_out[i]] : inner[a_red[i]];
@@ -571,6 +628,9 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
       t.b_off = b.t->locate(bid.data());
       a.t->block_dims(aid.data(), t.adims);
       b.t->block_dims(bid.data(), t.bdims);
+      t.pos = (int32_t) gchunks;
+      gchunks += task_chunks(lc, t);
+      TB_EXPECTS(gchunks < (1ll << 31), "contraction too long");
       // an admitted task over an exactly-zero block of a read-only operand, or over a
       // block that an earlier assignment of the same op list left without any
       // contribution, adds exactly zero to C: it is counted, not run
@@ -585,6 +645,7 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
     TB_EXPECTS(wl->tasks.size() < (1ull << 31), "too many tasks in one contraction");
     g.task_end = (int32_t) wl->tasks.size();
     wl->groups.push_back(g);
+    wl->group_chunks.push_back((int32_t) gchunks);
     skip_flops.push_back(gskip);
     skip_count.push_back(gskipn);
   } while(!cid.empty() && next_tuple(itval, c_nt));
@@ -600,6 +661,7 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
       for(int t = wl->groups[gi].task_begin; t < wl->groups[gi].task_end; t++) mine->tasks.push_back(wl->tasks[t]);
       g.task_end = (int32_t) mine->tasks.size();
       mine->groups.push_back(g);
+      mine->group_chunks.push_back(wl->group_chunks[gi]);
     }
     wl = mine;
   }
@@ -1140,12 +1202,12 @@ static std::shared_ptr<EnergySpec> build_energy(const Op& op, const LabelClasses
                  "orbital energies shorter than the index space");
       est[gi * nc + m] = (int32_t) first;
     }
-    // partial sums: 8 warps per output tile, tiles at least 128 x 48 (every kernel's)
+    // partial sums: 8 warps per output tile of at least 128 x 48, or 4 per tile of 64 x 32
     int64_t M = 1, N = 1, Bt = 1;
     for(int j = 0; j < lc.nm; j++) M *= g.cdims[lc.m_c[j]];
     for(int j = 0; j < lc.nn; j++) N *= g.cdims[lc.n_c[j]];
     for(int j = 0; j < lc.nbatch; j++) Bt *= g.cdims[lc.batch_c[j]];
-    es->npart += 8 * Bt * ((M + 127) / 128) * ((N + 47) / 48);
+    es->npart += Bt * std::max(8 * ((M + 127) / 128) * ((N + 47) / 48), 4 * ((M + 63) / 64) * ((N + 31) / 32));
   }
   int32_t* d_est = nullptr;
   TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_est), sizeof(int32_t) * est.size()));

@@ -45,12 +45,12 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
   return ok != 0;
 }
 
-// Bounded wait on an mbarrier phase; on timeout sets *err (atomically, first code
-// wins) and returns false.
+// Bounded wait on an mbarrier phase; on timeout sets *err (device memory, or host memory
+// mapped to the device) and returns false.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
   for(uint32_t i = 0; i < kWaitLimit; i++)
     if(mbar_try_wait(bar, parity)) return true;
-  atomicCAS(err, 0, code);
+  *reinterpret_cast<volatile int*>(err) = code;
   return false;
 }
 
