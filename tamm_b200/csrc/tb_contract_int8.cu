@@ -27,8 +27,7 @@
 #include "tb_internal.hpp"
 #include "tb_runtime.hpp"
 #include "tb_sm100.cuh"
-
-#include <cuda_bf16.h>
+#include "tb_split.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -44,23 +43,9 @@ void launch_contract_fp64(const Plan&, const WorkList&, double, double, int, con
 namespace {
 using namespace sm100;
 
-constexpr int MT = 128; // UMMA M: output rows of a tile
-constexpr int KC = 32;  // bytes of K per pipeline stage (one INT8 MMA k-step)
 constexpr int kMaxSmem = 227 * 1024; // dynamic shared memory per CTA on sm_100
 constexpr int NEPI     = 256;           // epilogue threads of the default kernel (warps 2-9)
 constexpr int NTHREADS = 64 + NEPI;     // warp 0 producer, warp 1 MMA issuer, warps 2-9 epilogue
-
-// One operand block to split into digit slices.
-struct SplitBlock {
-  int64_t src_off; // element offset in the FP64 arena
-  int64_t dst_off; // byte offset of the block's slices in the scratch
-  int32_t exp_off; // first exponent (int32 per padded row)
-  int32_t id;      // index into the per-block max-exponent array
-  int32_t rows, K, rows_pad, K_pad, tile_rows;
-  int32_t nr, nk, kcontig;
-  int32_t rdim[kMaxClass], rstr[kMaxClass];
-  int32_t kdim[kMaxClass], kstr[kMaxClass];
-};
 
 struct I8Task {
   int64_t a_off, b_off; // byte offsets of the A / B block slices
@@ -100,489 +85,6 @@ __device__ __forceinline__ int32_t decomp(int32_t x, int n, const int32_t* dims,
     x = q;
   }
   return off;
-}
-
-// Offset of the k-th K element of a row: contiguous K (the inner labels are the
-// trailing modes, last one stride 1) needs no index arithmetic.
-__device__ __forceinline__ int32_t koff(const SplitBlock& b, int32_t k) {
-  return b.kcontig ? k : decomp(k, b.nk, b.kdim, b.kstr);
-}
-
-constexpr int kPadRow = -0x7fffffff; // shift marker of a padding row (no digits)
-
-// Row exponent e with |x| * 2^-e <= 127/128 for every x of the row, so that
-// round(x * 2^(8S-1-e)) has a leading balanced digit within [-127, 127].
-__device__ __forceinline__ int row_exponent(double mx) {
-  int e = 0;
-  if(mx > 0.0) {
-    const double f = frexp(mx, &e); // mx = f * 2^e, f in [0.5, 1)
-    if(f > 127.0 / 128.0) e += 1;
-  }
-  return e;
-}
-
-
-// round(x * 2^sh) + bias as a 64-bit word whose bytes are the balanced digits + 128.
-// For S <= 6 (|X| < 2^47) one FMA against 1.5 * 2^52 leaves the integer, rounded to
-// nearest even, in the low mantissa bits (2^52 + 2^51 + X); larger S convert directly.
-template<int S>
-__device__ __forceinline__ uint64_t digit_word(double x, double f, uint64_t bias) {
-  if constexpr(S <= 6) {
-    const uint64_t t = (uint64_t) __double_as_longlong(fma(x, f, 6755399441055744.0));
-    return t + (bias - ((uint64_t) 1075 << 52) - ((uint64_t) 1 << 51));
-  }
-  else return (uint64_t) __double2ll_rn(x * f) + bias;
-}
-
-// Split in one pass over HBM: persistent CTAs, each taking 8-row groups ("chunks") in
-// turn.  Phase 1, warp w streams row w
-// (16-byte loads from the row's first 16-byte boundary, eight in flight per lane) for
-// its max |x| and row exponent; phase 2 re-reads the 8 rows, now resident in L2, one
-// 8-row x 16-k core matrix per warp and step: thread (row r, quad q) turns k =
-// 4q..4q+3 into Y = round(x * 2^(8S-1-e)) + 0x80..80, whose plain base-256 bytes are
-// the balanced digits + 128.  The bytes of 4 values are gathered per slice with PRMT,
-// flipped back with one XOR and stored as one 4-byte word, so every warp store is a
-// contiguous 128-byte core matrix.  Phase 2's re-reads and the digit stores are marked
-// evict-first (streaming), so that the rows still waiting for their phase 2 keep L2.
-// Slice layout per 32-byte K chunk of a tile: [K half (16 bytes)][digit][row][16 bytes],
-// i.e. the S digits' core matrices of one K half follow each other, so that the digits
-// j0..j1 of a B tile form one UMMA operand of (j1 - j0 + 1) x NT rows.  Residency (four CTAs per SM at 64 registers)
-// bounds the rows held in L2 between the phases to 4 x 148 x 8 rows (87 MB at K =
-// 2304, within the 126 MB L2).
-//
-// BF (the BF16x3 mode, S = 2): the row is scaled by 2^-e and each value x cut into two
-// bf16 pieces, hi = bf16(x) and lo = bf16(x - hi) (round to nearest), in the same
-// layout with 2-byte elements: a 16-byte core-matrix row holds 8 values, thread
-// (row r, pair q) converts k = 2q, 2q+1 of an 8-value column.
-template<int S, bool BF>
-__global__ void __launch_bounds__(256) k_split_fused(const SplitBlock* __restrict__ blocks,
-                                                     const int32_t* __restrict__ chunk_begin, int nblocks,
-                                                     int nchunks,
-                                                     const double* __restrict__ src, uint8_t* __restrict__ dst,
-                                                     int32_t* __restrict__ exps, int32_t* __restrict__ blockmax) {
-  __shared__ int     s_sh[8];
-  __shared__ int32_t s_off[8];
-  const int          warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint64_t     bias = S >= 8 ? 0x8080808080808080ull : ((1ull << (8 * S)) - 1) / 255 * 128;
-  // Block of chunk c: the last block whose first chunk is <= c (empty blocks skipped).
-  // The next chunk of a CTA is usually a few blocks on, so each lane holds the first
-  // chunk of one of the 32 blocks after the current one, loaded one chunk ahead (the
-  // load is in flight while the current chunk is split); past them, a 32-way search
-  // with one ballot per step keeps chunk_begin[lo] <= c < chunk_begin[hi], the lanes
-  // probing lo + step .. lo + 32 step, of which those at or below c form a prefix.
-  auto probe = [&](int from) {
-    return from + 1 + lane < nblocks ? __ldg(chunk_begin + from + 1 + lane) : 0x7fffffff;
-  };
-  int lo = 0, next_first = probe(0); // chunk_begin[lo] <= c holds for every later c
-  for(int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-    int hi;
-    {
-      const int cnt = __popc(__ballot_sync(0xffffffffu, next_first <= c));
-      lo += cnt;
-      hi = cnt < 32 ? lo + 1 : nblocks; // a failed probe at lo + 1 bounds the block
-    }
-    while(hi - lo > 1) {
-      const int      step = (hi - lo + 31) >> 5, idx = lo + (lane + 1) * step;
-      const unsigned le   = __ballot_sync(0xffffffffu, idx < hi && __ldg(chunk_begin + idx) <= c);
-      const int      cnt  = __popc(le);
-      hi                  = min(hi, lo + (cnt + 1) * step);
-      lo += cnt * step;
-    }
-    const int2       ch = make_int2(lo, 8 * (c - __ldg(chunk_begin + lo)));
-    const SplitBlock b  = blocks[ch.x];
-    next_first          = probe(lo);
-    {
-      const int     row    = ch.y + warp;
-      const bool    live   = row < b.rows;
-      const int32_t rowoff = live ? decomp(row, b.nr, b.rdim, b.rstr) : 0;
-      double        mx     = 0.0;
-      if(live) {
-        const double* s = src + b.src_off + rowoff;
-        double        m[8];
-#pragma unroll
-        for(int x = 0; x < 8; x++) m[x] = 0.0;
-        if(b.kcontig) {
-          // 16-byte loads from the first 16-byte boundary of the row on
-          const int      p0 = (reinterpret_cast<uintptr_t>(s) & 15) ? 1 : 0;
-          const int      np = (b.K - p0) >> 1;
-          const double2* s2 = reinterpret_cast<const double2*>(s + p0);
-          int            k  = lane;
-          for(; k + 224 < np; k += 256) {
-            double2 t[8];
-#pragma unroll
-            for(int x = 0; x < 8; x++) t[x] = __ldg(s2 + k + 32 * x);
-#pragma unroll
-            for(int x = 0; x < 8; x++) m[x] = fmax(m[x], fmax(fabs(t[x].x), fabs(t[x].y)));
-          }
-          for(; k < np; k += 32) {
-            const double2 t = __ldg(s2 + k);
-            m[0]            = fmax(m[0], fmax(fabs(t.x), fabs(t.y)));
-          }
-          if(lane == 0 && p0) m[1] = fmax(m[1], fabs(__ldg(s)));
-          if(lane == 1 && p0 + 2 * np < b.K) m[1] = fmax(m[1], fabs(__ldg(s + b.K - 1)));
-        }
-        else
-          for(int k = lane; k < b.K; k += 32) m[0] = fmax(m[0], fabs(__ldg(s + koff(b, k))));
-#pragma unroll
-        for(int x = 0; x < 8; x++) mx = fmax(mx, m[x]);
-      }
-#pragma unroll
-      for(int o = 16; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-      if(lane == 0) {
-        const int e = row_exponent(mx);
-        s_sh[warp]  = live ? (BF ? -e : 8 * S - 1 - e) : kPadRow;
-        s_off[warp] = rowoff;
-        exps[b.exp_off + row] = e;
-        if(mx > 0.0) atomicMax(blockmax + b.id, e);
-      }
-    }
-    __syncthreads();
-    const int     r = lane >> 2, q = lane & 3; // row within the 8-row group, k quad
-    const int     sh   = s_sh[r];
-    const bool    live = sh != kPadRow;
-    const double* s    = src + b.src_off + s_off[r];
-    // 2^sh as two factors, so that no factor overflows for extreme row exponents
-    const double f1  = ldexp(1.0, live ? sh / 2 : 0), f2 = ldexp(1.0, live ? sh - sh / 2 : 0);
-    const int g8 = (ch.y % b.tile_rows) >> 3;
-    if constexpr(BF) {
-      const int nkc = b.K_pad * 2 / KC;
-      uint8_t*  out = dst + b.dst_off + (int64_t) (ch.y / b.tile_rows) * nkc * S * b.tile_rows * KC + g8 * 128 +
-                     r * 16 + q * 4;
-      const bool vec = live && b.kcontig && !(reinterpret_cast<uintptr_t>(s) & 15);
-      for(int k8 = warp; k8 < b.K_pad / 8; k8 += 8) {
-        const int k0 = k8 * 8 + q * 2;
-        double    v[2];
-        if(vec && k0 + 1 < b.K) {
-          const double2 v01 = __ldcs(reinterpret_cast<const double2*>(s + k0));
-          v[0] = v01.x, v[1] = v01.y;
-        }
-        else
-#pragma unroll
-          for(int x = 0; x < 2; x++) v[x] = (live && k0 + x < b.K) ? __ldcs(s + koff(b, k0 + x)) : 0.0;
-        uint32_t hi = 0, lo = 0;
-#pragma unroll
-        for(int x = 0; x < 2; x++) {
-          const double         y = v[x] * f1 * f2;
-          const __nv_bfloat16  h = __double2bfloat16(y);
-          const __nv_bfloat16  t = __double2bfloat16(y - (double) __bfloat162float(h));
-          hi |= (uint32_t) __bfloat16_as_ushort(h) << (16 * x);
-          lo |= (uint32_t) __bfloat16_as_ushort(t) << (16 * x);
-        }
-        uint8_t* o = out + (int64_t) (k8 >> 1) * S * b.tile_rows * KC + (k8 & 1) * S * b.tile_rows * 16;
-        __stcs(reinterpret_cast<unsigned int*>(o), hi);
-        __stcs(reinterpret_cast<unsigned int*>(o + b.tile_rows * 16), lo);
-      }
-    }
-    else {
-      const int    nkc = b.K_pad / KC;
-      uint8_t* out = dst + b.dst_off + (int64_t) (ch.y / b.tile_rows) * nkc * S * b.tile_rows * KC + g8 * 128 + r * 16 +
-                     q * 4;
-      const bool vec = live && b.kcontig && !(reinterpret_cast<uintptr_t>(s) & 15);
-      // loads of one 16-value column (this thread's row and quad) and the conversion
-      // of it into S 4-byte digit words; two columns per iteration keep the second
-      // column's loads in flight while the first converts
-      auto load4 = [&](int k16, double (&v)[4]) {
-        const int k0 = k16 * 16 + q * 4;
-        if(vec && k0 + 3 < b.K) {
-          const double2 v01 = __ldcs(reinterpret_cast<const double2*>(s + k0));
-          const double2 v23 = __ldcs(reinterpret_cast<const double2*>(s + k0 + 2));
-          v[0] = v01.x, v[1] = v01.y, v[2] = v23.x, v[3] = v23.y;
-        }
-        else
-#pragma unroll
-          for(int x = 0; x < 4; x++) {
-            const int k = k0 + x;
-            v[x]        = (live && k < b.K) ? __ldcs(s + koff(b, k)) : 0.0;
-          }
-      };
-      auto emit = [&](int k16, const double (&v)[4]) {
-        uint32_t lo[4], hi[4];
-#pragma unroll
-        for(int x = 0; x < 4; x++) {
-          const uint64_t Y = digit_word<S>(v[x] * f2, f1, bias);
-          lo[x]            = (uint32_t) Y;
-          hi[x]            = (uint32_t) (Y >> 32);
-        }
-        uint8_t* o = out + (int64_t) (k16 >> 1) * S * b.tile_rows * KC + (k16 & 1) * S * b.tile_rows * 16;
-#pragma unroll
-        for(int i = 0; i < S; i++) {
-          const int p = S - 1 - i; // byte of Y holding digit i
-          uint32_t  w;
-          if(p < 4) {
-            const uint32_t t0 = __byte_perm(lo[0], lo[1], p | ((p + 4) << 4));
-            const uint32_t t1 = __byte_perm(lo[2], lo[3], p | ((p + 4) << 4));
-            w                 = __byte_perm(t0, t1, 0x5410);
-          }
-          else {
-            const uint32_t t0 = __byte_perm(hi[0], hi[1], (p - 4) | (p << 4));
-            const uint32_t t1 = __byte_perm(hi[2], hi[3], (p - 4) | (p << 4));
-            w                 = __byte_perm(t0, t1, 0x5410);
-          }
-          __stcs(reinterpret_cast<unsigned int*>(o + (int64_t) i * b.tile_rows * 16), w ^ 0x80808080u);
-        }
-      };
-      const int n16 = b.K_pad / 16;
-      for(int k16 = warp; k16 < n16; k16 += 16) {
-        double v0[4], v1[4];
-        load4(k16, v0);
-        const bool two = k16 + 8 < n16;
-        if(two) load4(k16 + 8, v1);
-        emit(k16, v0);
-        if(two) emit(k16 + 8, v1);
-      }
-    }
-    __syncthreads(); // s_sh / s_off are rewritten for the next chunk
-  }
-}
-
-// Staged split for operand blocks whose rows lie one after another in memory (K
-// contiguous and row r at element offset r * K: e.g. v(a,b,c,d) split as rows (a,b) by
-// K = (c,d)).  The unit of work is a pair of rows, one contiguous range of 2K doubles,
-// brought into shared memory by one bulk copy; every element is read from HBM once, and
-// both the row maxima and the digit conversion read shared memory.
-//   Producer (warp 0): resolves 32 units at a time, one per lane (block by binary
-// search over the per-block chunk prefix, then the unit's copy range and the fields the
-// consumers need), and issues their copies in order into the stage of the group that
-// takes each unit.  A CTA owns whole 8-row chunks: the four units of a chunk fill the
-// same 128-byte lines of every digit plane, and lines completed by one SM within a
-// short time leave L2 whole (units spread over SMs measured 1.4x slower at the size
-// of the O=40/V=360 ladder's v, while as fast on a quarter of it).  The unit records
-// travel in shared memory beside the stages, so a consumer reads no block record from
-// global memory.
-//   Consumers: independent groups of kSplitGroup warps, each group with two stages of
-// its own, so a group's only synchronisation is a named barrier of its own warps.
-// Warp h of a group takes the h-th K range of the row maxima and every kSplitGroup-th
-// group of four 16-k chunks of the digits.  Lane (row, chunk c, quad q) reads its four
-// values in an order rotated by (q + c) mod 4, so that the 16 lanes of a row hit 16
-// distinct bank pairs, and the final byte permute puts the digits back in k order;
-// each warp store covers the two rows of 32-byte sectors.
-//   The copy covers the 16-byte aligned interior [floor16(start), floor16(end)) of the
-// pair; a last element past floor16(end) is loaded with a plain load.  Units made of
-// padding rows only write their exponents.  Waits are bounded: a timeout records
-// `code` in *err and the warps of a group agree (bar.red) to leave together.
-struct UnitMeta {
-  int64_t tail_src; // element index of the unit's last element (the tail load)
-  int64_t dst_off;  // byte offset of the block's digits
-  int32_t exp_base; // exponent index of the unit's first row
-  int32_t id, K, K_pad, tile_rows, row0, nlive, delta, tail;
-  int32_t pad[3];
-};
-static_assert(sizeof(UnitMeta) == 64, "unit record size");
-
-constexpr int     kSplitGroup     = 4;            // consumer warps per group
-constexpr int     kSplitMaxGroups = 4;            // groups per CTA, at most
-constexpr int64_t kStagedSmem     = 227 * 1024;   // dynamic shared memory of one CTA, at most
-constexpr int64_t kStagedHead     = 2048;         // barriers, unit records, partial maxima
-// bytes of one stage of 2 rows of K doubles (+16 for the aligned start), 128-byte multiple
-__host__ __device__ constexpr int64_t staged_stage_bytes(int64_t K) {
-  return (2 * K * 8 + 16 + 127) / 128 * 128;
-}
-
-// TR: rows per operand tile (128 for A; 0 = read from the unit record).
-template<int S, int TR>
-__global__ void __launch_bounds__(32 * (1 + kSplitMaxGroups * kSplitGroup), 1)
-  k_split_staged(const SplitBlock* __restrict__ blocks, const int32_t* __restrict__ chunk_begin, int nblocks,
-                 int nchunks, int ngroups, uint32_t stage_bytes, const double* __restrict__ src,
-                 uint8_t* __restrict__ dst, int32_t* __restrict__ exps, int32_t* __restrict__ blockmax, int* err) {
-  constexpr int G = kSplitGroup;
-  extern __shared__ __align__(128) uint8_t sm[];
-  uint64_t*     full  = reinterpret_cast<uint64_t*>(sm);           // [2 per group]
-  uint64_t*     empty = full + 2 * kSplitMaxGroups;                // [2 per group]
-  UnitMeta*     meta  = reinterpret_cast<UnitMeta*>(sm + 256);     // [2 per group]
-  double*       part  = reinterpret_cast<double*>(sm + 1280);      // [group][parity][warp][row]
-  uint8_t*      ring  = sm + kStagedHead;
-  static_assert(4 * kSplitMaxGroups * 8 <= 256 && 256 + 2 * kSplitMaxGroups * 64 <= 1280, "stage records");
-  static_assert(1280 + 2 * kSplitMaxGroups * G * 2 * 8 <= kStagedHead, "partial maxima");
-  const int     warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int     nunits = nchunks * 4; // two rows per unit, four units per 8-row chunk
-  // units of this CTA: the four of each of its chunks
-  const int     myunits = ((nchunks - (int) blockIdx.x + (int) gridDim.x - 1) / (int) gridDim.x) * 4;
-  if(threadIdx.x == 0) {
-    for(int x = 0; x < 2 * ngroups; x++) {
-      mbar_init(&full[x], 1);
-      mbar_init(&empty[x], G); // one arrival per warp of the group
-    }
-    fence_mbarrier_init();
-  }
-  __syncthreads();
-  if(warp == 0) {
-    // ---------------- producer: 32 unit records at a time, copies in unit order -------
-    // The CTA's j-th unit is unit j mod 4 of 8-row chunk blockIdx.x + (j / 4) * gridDim.x
-    // (the four units of a chunk, whose digits share every 128-byte line, are written
-    // by one SM close together in time); it goes to group j mod ngroups, that group's
-    // stage (j / ngroups) mod 2.
-    for(int jb = 0; jb < myunits; jb += 32) {
-      const int jl = jb + lane;
-      const int u  = jl < myunits ? ((int) blockIdx.x + (jl >> 2) * (int) gridDim.x) * 4 + (jl & 3) : nunits;
-      UnitMeta  mine{};
-      uintptr_t a16   = 0;
-      uint32_t  bytes = 0;
-      if(u < nunits) {
-        const int c = u >> 2;
-        int       lo = 0, hi = nblocks - 1; // last block whose first chunk is <= c
-        while(lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if(__ldg(chunk_begin + mid) <= c) lo = mid;
-          else hi = mid - 1;
-        }
-        const SplitBlock& b    = blocks[lo];
-        const int         row0 = 8 * (c - __ldg(chunk_begin + lo)) + (u & 3) * 2;
-        const int         K    = b.K;
-        const int         nl   = max(0, min(2, b.rows - row0));
-        mine.dst_off   = b.dst_off;
-        mine.exp_base  = b.exp_off + row0;
-        mine.id        = b.id;
-        mine.K         = K;
-        mine.K_pad     = b.K_pad;
-        mine.tile_rows = b.tile_rows;
-        mine.row0      = row0;
-        mine.nlive     = nl;
-        mine.tail_src  = b.src_off + (int64_t) (row0 + nl) * K - 1;
-        if(nl > 0) {
-          const uintptr_t start = reinterpret_cast<uintptr_t>(src + b.src_off + (int64_t) row0 * K);
-          const uintptr_t end   = start + (uintptr_t) nl * K * 8;
-          a16                   = start & ~uintptr_t(15);
-          bytes                 = (uint32_t) ((end & ~uintptr_t(15)) - a16);
-          mine.delta            = (int32_t) (start - a16);
-          mine.tail             = (end & 15) ? 1 : 0;
-        }
-      }
-      for(int t = 0; t < 32; t++) {
-        if(jb + t >= myunits) break;
-        const int      j     = jb + t;
-        const int      x     = 2 * (j % ngroups) + ((j / ngroups) & 1);
-        const uint32_t round = (uint32_t) (j / (2 * ngroups));
-        if(!mbar_wait(&empty[x], (round & 1) ^ 1, err, 21)) return; // (every lane polls; all agree)
-        if(lane == t) {
-          meta[x] = mine;
-          mbar_arrive_expect_tx(&full[x], bytes);
-          if(bytes > 0)
-            bulk_g2s(ring + (size_t) x * stage_bytes, reinterpret_cast<const void*>(a16), bytes, &full[x]);
-        }
-        __syncwarp();
-      }
-    }
-    return;
-  }
-  // ---------------- consumers: groups of G warps ----------------
-  const int cw = warp - 1, grp = cw / G, h = cw % G;
-  if(grp >= ngroups) return;
-  const int      barid = 1 + grp; // named barrier of the group (0 is __syncthreads)
-  const uint64_t bias  = S >= 8 ? 0x8080808080808080ull : ((1ull << (8 * S)) - 1) / 255 * 128;
-  const int      rr = lane >> 4, c = (lane >> 2) & 3, q = lane & 3; // row of the pair, chunk, quad
-  const int      rot = (q + c) & 3;
-  uint32_t       sel2 = 0; // byte permute taking the rotated values back to k order
-#pragma unroll
-  for(int pos = 0; pos < 4; pos++) {
-    const int t = (pos - rot) & 3;
-    sel2 |= (uint32_t) (t < 2 ? t : t + 2) << (4 * pos);
-  }
-  for(int j = grp; j < myunits; j += ngroups) {
-    const int      par   = (j / ngroups) & 1, x = 2 * grp + par;
-    const uint32_t round = (uint32_t) (j / (2 * ngroups));
-    {
-      const bool got = mbar_wait(&full[x], round & 1, err, 22);
-      uint32_t   anyfail;
-      asm volatile("{\n\t.reg .pred p, q;\n\tsetp.eq.u32 p, %1, 0;\n\t"
-                   "bar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
-                   : "=r"(anyfail)
-                   : "r"((uint32_t) got), "r"(barid), "n"(32 * G)
-                   : "memory");
-      if(anyfail) return;
-    }
-    const UnitMeta m       = meta[x];
-    const int      K       = m.K;
-    const int      tr      = TR > 0 ? TR : m.tile_rows;
-    double*        rowbase = reinterpret_cast<double*>(ring + (size_t) x * stage_bytes + m.delta);
-    if(m.tail) { // the last element, past the copy's 16-byte aligned end
-      if(h == 0 && lane == 0) {
-        rowbase[(int64_t) m.nlive * K - 1] = __ldg(src + m.tail_src);
-        // ordered before the bulk copy that later refills this stage
-        asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
-      }
-      asm volatile("bar.sync %0, %1;\n" ::"r"(barid), "n"(32 * G) : "memory");
-    }
-    // row maxima: 16 lanes per row over this warp's K range, then over the group
-    const double* xr   = rowbase + (int64_t) rr * K;
-    const bool    live = rr < m.nlive;
-    double        mx   = 0.0;
-    if(live) {
-      const int span = (K + G - 1) / G, kb = h * span, ke = min(K, kb + span);
-      double    m0 = 0.0, m1 = 0.0, m2 = 0.0, m3 = 0.0;
-      int       k = kb + (lane & 15);
-      for(; k + 48 < ke; k += 64) {
-        m0 = fmax(m0, fabs(xr[k]));
-        m1 = fmax(m1, fabs(xr[k + 16]));
-        m2 = fmax(m2, fabs(xr[k + 32]));
-        m3 = fmax(m3, fabs(xr[k + 48]));
-      }
-      for(; k < ke; k += 16) m0 = fmax(m0, fabs(xr[k]));
-      mx = fmax(fmax(m0, m1), fmax(m2, m3));
-    }
-#pragma unroll
-    for(int o = 8; o > 0; o >>= 1) mx = fmax(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    // partials alternate between two buffers by unit parity: a warp writes this buffer
-    // again only after the group's next barrier, which every reader of it has passed
-    double* pp = part + (grp * 2 + par) * G * 2;
-    if((lane & 15) == 0) pp[h * 2 + rr] = mx;
-    asm volatile("bar.sync %0, %1;\n" ::"r"(barid), "n"(32 * G) : "memory");
-    mx = 0.0;
-#pragma unroll
-    for(int w = 0; w < G; w++) mx = fmax(mx, pp[w * 2 + rr]);
-    const int e = row_exponent(mx);
-    if(h == 0 && (lane & 15) == 0) {
-      exps[m.exp_base + rr] = e;
-      if(mx > 0.0) atomicMax(blockmax + m.id, e);
-    }
-    if(m.nlive > 0) {
-      // digits: 2^sh in one factor where it is a normal double, else as two (tiny rows)
-      const int     sh   = live ? 8 * S - 1 - e : 0;
-      const bool    wide = sh > 1000 || sh < -1000;
-      const double  f1 = ldexp(1.0, wide ? sh / 2 : sh), f2 = ldexp(1.0, wide ? sh - sh / 2 : 0);
-      const int     row   = m.row0 + rr;
-      const int     nkc   = m.K_pad / KC;
-      const int64_t dstep = (int64_t) S * tr * 16; // one K half of a 32-byte K chunk
-      uint8_t*      o = dst + m.dst_off + (int64_t) (row / tr) * nkc * S * tr * KC + ((row % tr) >> 3) * 128 +
-                   (row & 7) * 16 + q * 4 + ((c >> 1) * 2 + (c & 1) + (int64_t) h * 4) * dstep;
-      const int     n16     = m.K_pad / 16;
-      const bool    anywide = __any_sync(0xffffffffu, wide && live);
-      for(int k16 = 4 * h + c; k16 < n16; k16 += 4 * G, o += 4 * G * dstep) {
-        const int k0 = k16 * 16 + q * 4;
-        double    v[4];
-#pragma unroll
-        for(int t = 0; t < 4; t++) {
-          const int kk = k0 + ((t + rot) & 3);
-          v[t]         = (live && kk < K) ? xr[kk] : 0.0;
-        }
-        if(anywide)
-#pragma unroll
-          for(int t = 0; t < 4; t++) v[t] *= f2;
-        uint32_t lo[4], hi[4];
-#pragma unroll
-        for(int t = 0; t < 4; t++) {
-          const uint64_t Y = digit_word<S>(v[t], f1, bias);
-          lo[t]            = (uint32_t) Y;
-          hi[t]            = (uint32_t) (Y >> 32);
-        }
-#pragma unroll
-        for(int i = 0; i < S; i++) {
-          const int p = S - 1 - i; // byte of Y holding digit i
-          uint32_t  t0, t1;
-          if(p < 4) {
-            t0 = __byte_perm(lo[0], lo[1], p | ((p + 4) << 4));
-            t1 = __byte_perm(lo[2], lo[3], p | ((p + 4) << 4));
-          }
-          else {
-            t0 = __byte_perm(hi[0], hi[1], (p - 4) | (p << 4));
-            t1 = __byte_perm(hi[2], hi[3], (p - 4) | (p << 4));
-          }
-          __stcs(reinterpret_cast<unsigned int*>(o + (int64_t) i * tr * 16), __byte_perm(t0, t1, sel2) ^ 0x80808080u);
-        }
-      }
-    }
-    __syncwarp();
-    if(lane == 0) mbar_arrive(&empty[x]); // this warp is done with the stage
-  }
 }
 
 // Slice count per task: a task whose largest possible product (2^(maxexp A + maxexp
@@ -1203,16 +705,6 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
 
 // ---------------------------------------------------------------- host side
 
-// Blocks split by one kernel: the staged kernel (rows contiguous) or the general one,
-// with their chunk table (first 8-row chunk of each block, then the total).
-struct SplitSet {
-  std::vector<SplitBlock> blocks;
-  std::vector<int32_t>    cbegin;
-  SplitBlock*             d_blocks = nullptr;
-  int32_t*                d_cbegin = nullptr;
-  int                     kmax     = 0;
-};
-
 // Digits of every stored, nonzero block of a read-only tensor under one operand view
 // (side, digit count, tile rows, element size, the label classes' rows / K of the
 // tensor's modes), kept in the context's arena while the tensor stays read-only, so
@@ -1254,7 +746,6 @@ struct DigitEntry final : DigitCacheEntry {
 struct I8Layout {
   int                     S = 0, NT = 0, esize = 1; // digits, output tile width, bytes per digit
   std::vector<SplitBlock> a_blocks, b_blocks;
-  std::vector<int32_t>    a_cbegin, b_cbegin; // first 8-row chunk of each block, then the total
   // the blocks of each operand split by the staged kernel (rows contiguous) and by the
   // general one, each with its own chunk table
   SplitSet                a_staged, a_general, b_staged, b_general;
@@ -1267,10 +758,6 @@ struct I8Layout {
   int64_t                 nexp = 0, a_nexp = 0;
   double                  int8_ops = 0;
   double                  kc_per_item = 0; // mean 32-byte K steps of an output tile (all its tasks)
-  SplitBlock*             d_ablocks = nullptr;
-  SplitBlock*             d_bblocks = nullptr;
-  int32_t*                d_acbegin = nullptr;
-  int32_t*                d_bcbegin = nullptr;
   I8Task*                 d_tasks   = nullptr;
   I8Item*                 d_items   = nullptr;
   I8TaskMeta*             d_meta    = nullptr;
@@ -1286,10 +773,6 @@ struct I8Layout {
         cudaFree(x->d_blocks);
         cudaFree(x->d_cbegin);
       }
-      cudaFree(d_ablocks);
-      cudaFree(d_bblocks);
-      cudaFree(d_acbegin);
-      cudaFree(d_bcbegin);
       cudaFree(d_tasks);
       cudaFree(d_items);
       cudaFree(d_meta);
@@ -1304,73 +787,6 @@ struct I8Layout {
 int nt_for(int S) { return S <= 6 ? 80 : 64; }
 
 int64_t rup(int64_t x, int64_t m) { return (x + m - 1) / m * m; }
-
-// The GEMM view of one operand block: rows = the outer labels (positions rpos, in C's
-// order), K = the inner labels (positions kpos, in A's order), element strides of the
-// block's row-major layout; tile_rows / kstep set the padding.
-SplitBlock view_block(const int32_t* dims, int nmodes, const int8_t* rpos, int nr, const int8_t* kpos, int nk,
-                      int tile_rows, int kstep) {
-  int64_t str[kMaxModes];
-  int64_t st = 1;
-  for(int i = nmodes - 1; i >= 0; i--) {
-    str[i] = st;
-    st *= dims[i];
-  }
-  SplitBlock b{};
-  b.nr   = nr;
-  b.nk   = nk;
-  b.rows = 1;
-  for(int j = 0; j < nr; j++) {
-    b.rdim[j] = dims[rpos[j]];
-    b.rstr[j] = (int32_t) str[rpos[j]];
-    b.rows *= b.rdim[j];
-  }
-  b.K = 1;
-  for(int j = 0; j < nk; j++) {
-    b.kdim[j] = dims[kpos[j]];
-    b.kstr[j] = (int32_t) str[kpos[j]];
-    b.K *= b.kdim[j];
-  }
-  b.kcontig = 1;
-  for(int j = 0; j < nk; j++) b.kcontig &= (kpos[j] == nmodes - nk + j) ? 1 : 0;
-  b.tile_rows = tile_rows;
-  b.rows_pad  = (int32_t) rup(b.rows, tile_rows);
-  b.K_pad     = (int32_t) rup(b.K, kstep);
-  return b;
-}
-
-// Staged-kernel eligibility: K contiguous, row r at element offset r * K, and the two
-// stages of one warp group (two rows each) fit in shared memory.
-bool staged_ok(const SplitBlock& b, int esize) {
-  if(esize != 1 || !b.kcontig) return false;
-  int64_t st = b.K;
-  for(int j = b.nr - 1; j >= 0; j--) {
-    if(b.rstr[j] != st) return false;
-    st *= b.rdim[j];
-  }
-  return staged_stage_bytes(b.K) * 2 + kStagedHead <= kStagedSmem;
-}
-
-void chunk_table(const std::vector<SplitBlock>& bl, std::vector<int32_t>& out) {
-  out.resize(bl.size() + 1);
-  int64_t n = 0;
-  for(size_t i = 0; i < bl.size(); i++) {
-    out[i] = (int32_t) n;
-    n += bl[i].rows_pad / 8;
-  }
-  TB_EXPECTS(n < (1ll << 31), "too many split row groups");
-  out[bl.size()] = (int32_t) n;
-}
-
-void partition_sets(const std::vector<SplitBlock>& all, int esize, SplitSet& st, SplitSet& ge) {
-  for(const auto& b: all) {
-    SplitSet& x = staged_ok(b, esize) ? st : ge;
-    x.blocks.push_back(b);
-    x.kmax = std::max(x.kmax, b.K);
-  }
-  chunk_table(st.blocks, st.cbegin);
-  chunk_table(ge.blocks, ge.cbegin);
-}
 
 template<typename T>
 void upload_vec(T*& dptr, const std::vector<T>& vec) {
@@ -1469,19 +885,8 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
   L->slice_bytes = abytes + bbytes;
   L->a_nexp      = aexp;
   L->nexp        = aexp + bexp;
-  auto chunks    = [](const std::vector<SplitBlock>& bl, std::vector<int32_t>& out) {
-    out.resize(bl.size() + 1);
-    int64_t n = 0;
-    for(size_t i = 0; i < bl.size(); i++) {
-      out[i] = (int32_t) n;
-      n += bl[i].rows_pad / 8;
-    }
-    out[bl.size()] = (int32_t) n;
-  };
-  chunks(L->a_blocks, L->a_cbegin);
-  chunks(L->b_blocks, L->b_cbegin);
-  partition_sets(L->a_blocks, esize, L->a_staged, L->a_general);
-  partition_sets(L->b_blocks, esize, L->b_staged, L->b_general);
+  partition_sets(L->a_blocks, L->a_staged, L->a_general);
+  partition_sets(L->b_blocks, L->b_staged, L->b_general);
   // Output tiles, longest group first (every tile of a group costs the same, so
   // ordering the groups orders the tiles).  Among groups of equal work, those whose
   // first task reads the same A block (the same rows: e.g. W(a,b,c,..) = v(b,c,..) *
@@ -1542,14 +947,10 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
     TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&dptr), sizeof(T) * vec.size()));
     TB_CUDA(cudaMemcpy(dptr, vec.data(), sizeof(T) * vec.size(), cudaMemcpyHostToDevice));
   };
-  up(L->d_ablocks, L->a_blocks);
-  up(L->d_bblocks, L->b_blocks);
   for(SplitSet* x: {&L->a_staged, &L->a_general, &L->b_staged, &L->b_general}) {
     up(x->d_blocks, x->blocks);
     up(x->d_cbegin, x->cbegin);
   }
-  up(L->d_acbegin, L->a_cbegin);
-  up(L->d_bcbegin, L->b_cbegin);
   up(L->d_tasks, L->tasks);
   up(L->d_items, L->items);
   up(L->d_meta, L->meta);
@@ -1569,46 +970,6 @@ int sm_count() {
   return n;
 }
 
-template<int S, int TR>
-void launch_staged(const SplitSet& x, const double* src, uint8_t* slices, int32_t* exps,
-                   int32_t* blockmax, int* err, cudaStream_t st) {
-  const int      nblocks = (int) x.cbegin.size() - 1, nchunks = x.cbegin.back();
-  const uint32_t sb      = (uint32_t) staged_stage_bytes(x.kmax);
-  const int      ngroups = (int) std::min<int64_t>(kSplitMaxGroups, (kStagedSmem - kStagedHead) / (2 * (int64_t) sb));
-  TB_EXPECTS(ngroups >= 1, "staged split: one group's stages must fit in shared memory");
-  const size_t   smem    = kStagedHead + (size_t) 2 * ngroups * sb;
-  static bool    configured[64] = {false};
-  int            dev            = 0;
-  TB_CUDA(cudaGetDevice(&dev));
-  if(dev < 64 && !configured[dev]) {
-    TB_CUDA(cudaFuncSetAttribute(k_split_staged<S, TR>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStagedSmem));
-    configured[dev] = true;
-  }
-  const int grid = (int) std::min<int64_t>((int64_t) nchunks, sm_count()); // whole chunks per CTA
-  k_split_staged<S, TR><<<grid, 32 * (1 + ngroups * kSplitGroup), smem, st>>>(
-    x.d_blocks, x.d_cbegin, nblocks, nchunks, ngroups, sb, src, slices, exps, blockmax, err);
-}
-
-// Splits the blocks of one operand: the staged kernel for the blocks with contiguous
-// rows, the general kernel for the rest.
-template<int S, bool BF>
-void split_sets(const SplitSet& staged, const SplitSet& general, const double* src, uint8_t* slices,
-                int32_t* exps, int32_t* blockmax, int* err, cudaStream_t st) {
-  if(!general.blocks.empty() && general.cbegin.back() > 0) {
-    const int nblocks = (int) general.cbegin.size() - 1, nchunks = general.cbegin.back();
-    k_split_fused<S, BF><<<std::min(nchunks, sm_count() * 8), 256, 0, st>>>(general.d_blocks, general.d_cbegin,
-                                                                            nblocks, nchunks, src, slices, exps,
-                                                                            blockmax);
-  }
-  if constexpr(!BF) {
-    if(!staged.blocks.empty() && staged.cbegin.back() > 0) {
-      // A tiles (128 rows) with the row count fixed at compile time, B tiles read it
-      if(staged.blocks.front().tile_rows == MT) launch_staged<S, MT>(staged, src, slices, exps, blockmax, err, st);
-      else launch_staged<S, 0>(staged, src, slices, exps, blockmax, err, st);
-    }
-  }
-}
-
 template<int S, bool BF>
 void launch_split(const I8Layout& L, const WorkList& wl, const double* A, const double* B, uint8_t* slices,
                   int32_t* exps, cudaStream_t st) {
@@ -1616,13 +977,13 @@ void launch_split(const I8Layout& L, const WorkList& wl, const double* A, const 
   for(DigitEntry* e: {L.a_cache.get(), L.b_cache.get()})
     if(e && !e->filled) {
       TB_CUDA(cudaMemsetAsync(e->blockmax, 0x80, sizeof(int32_t) * std::max<size_t>(e->by_off.size(), 1), st));
-      split_sets<S, BF>(e->staged, e->general, e->src, e->slices, e->exps, e->blockmax, e->err, st);
+      split_sets(S, BF, e->staged, e->general, e->src, e->slices, e->exps, e->blockmax, e->err, st);
       e->filled = true;
     }
   // 0x80808080: below every exponent sum, marks blocks without a nonzero row
   TB_CUDA(cudaMemsetAsync(L.d_blockmax, 0x80, sizeof(int32_t) * (L.a_blocks.size() + L.b_blocks.size()), st));
-  split_sets<S, BF>(L.a_staged, L.a_general, A, slices, exps, L.d_blockmax, L.d_err, st);
-  split_sets<S, BF>(L.b_staged, L.b_general, B, slices, exps, L.d_blockmax, L.d_err, st);
+  split_sets(S, BF, L.a_staged, L.a_general, A, slices, exps, L.d_blockmax, L.d_err, st);
+  split_sets(S, BF, L.b_staged, L.b_general, B, slices, exps, L.d_blockmax, L.d_err, st);
   const int ng = (int) wl.groups.size();
   if constexpr(BF) { // both bf16 pieces in every task
     if(!L.tasks.empty()) TB_CUDA(cudaMemsetAsync(L.d_tslices, S, L.tasks.size(), st));
@@ -1783,7 +1144,7 @@ std::shared_ptr<DigitEntry> digit_entry(const Plan& plan, const Tensor* T, int s
   *e->used += total;
   TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&e->err), sizeof(int)));
   TB_CUDA(cudaMemset(e->err, 0, sizeof(int)));
-  partition_sets(all, esize, e->staged, e->general);
+  partition_sets(all, e->staged, e->general);
   for(SplitSet* x: {&e->staged, &e->general}) {
     upload_vec(x->d_blocks, x->blocks);
     upload_vec(x->d_cbegin, x->cbegin);
@@ -1985,7 +1346,7 @@ __global__ void k_noalloc_setup(NoAllocDesc d, unsigned char* base) {
   }
   I8Item* items = reinterpret_cast<I8Item*>(base + kCtlItems);
   for(int i = tid; i < d.mtiles * d.ntiles; i += nth) items[i] = I8Item{0, i / d.ntiles, i % d.ntiles, 0};
-  if(tid == 0) { // one block per operand: first chunk 0, then the chunk count
+  if(tid == 0) { // one block per operand: first unit 0, then the unit count
     int32_t* cb = reinterpret_cast<int32_t*>(base + d.chunks_off);
     cb[0] = 0, cb[1] = d.nchunk_a, cb[2] = 0, cb[3] = d.nchunk_b;
   }
@@ -2006,9 +1367,8 @@ void noalloc_launch(const NoAllocDesc& d, unsigned char* base, int64_t exps_off,
   int32_t*      exps = reinterpret_cast<int32_t*>(base + exps_off);
   uint8_t*      sl   = base + slices_off;
   k_noalloc_setup<<<8, 256, 0, st>>>(d, base);
-  const int cap = sm_count() * 8;
-  k_split_fused<S, false><<<std::min(d.nchunk_a, cap), 256, 0, st>>>(sb, cb, 1, d.nchunk_a, A, sl, exps, bmax);
-  k_split_fused<S, false><<<std::min(d.nchunk_b, cap), 256, 0, st>>>(sb + 1, cb + 2, 1, d.nchunk_b, B, sl, exps, bmax);
+  split_one(S, d.a, sb, cb, A, sl, exps, bmax, st);
+  split_one(S, d.b, sb + 1, cb + 2, B, sl, exps, bmax, st);
   k_task_slices<<<1, 32, 0, st>>>(meta, grp, 1, bmax, bmax, S, tsl);
   I8Params p{};
   p.a_slices = sl;
@@ -2066,39 +1426,18 @@ extern "C" int tb_block_multiply_int8_noalloc(double alpha, const double* a, con
     const int S  = nslices > 0 ? nslices : slices_for(1e-11);
     const int NT = S <= 6 ? 80 : 64;
 
-    // block geometry, the same views the allocating path builds (build_layout)
-    int64_t astr[kMaxModes], bstr[kMaxModes];
-    {
-      int64_t s = 1;
-      for(int i = na - 1; i >= 0; i--) {
-        astr[i] = s;
-        s *= adims[i];
-      }
-      s = 1;
-      for(int i = nb - 1; i >= 0; i--) {
-        bstr[i] = s;
-        s *= bdims[i];
-      }
-    }
     NoAllocDesc d{};
     int64_t     M = 1, N = 1, K = 1;
     for(int j = 0; j < lc.nm; j++) {
       TB_EXPECTS(cdims[lc.m_c[j]] == adims[lc.m_a[j]], "A-outer label extents differ (C vs A)");
-      d.a.rdim[j] = (int32_t) adims[lc.m_a[j]];
-      d.a.rstr[j] = (int32_t) astr[lc.m_a[j]];
       M *= adims[lc.m_a[j]];
     }
     for(int j = 0; j < lc.nn; j++) {
       TB_EXPECTS(cdims[lc.n_c[j]] == bdims[lc.n_b[j]], "B-outer label extents differ (C vs B)");
-      d.b.rdim[j] = (int32_t) bdims[lc.n_b[j]];
-      d.b.rstr[j] = (int32_t) bstr[lc.n_b[j]];
       N *= bdims[lc.n_b[j]];
     }
     for(int j = 0; j < lc.nk; j++) {
       TB_EXPECTS(adims[lc.k_a[j]] == bdims[lc.k_b[j]], "inner label extents differ (A vs B)");
-      d.a.kdim[j] = d.b.kdim[j] = (int32_t) adims[lc.k_a[j]];
-      d.a.kstr[j] = (int32_t) astr[lc.k_a[j]];
-      d.b.kstr[j] = (int32_t) bstr[lc.k_b[j]];
       K *= adims[lc.k_a[j]];
     }
     TB_EXPECTS(M * K < (1ll << 31) && N * K < (1ll << 31) && M * N < (1ll << 31),
@@ -2115,32 +1454,15 @@ extern "C" int tb_block_multiply_int8_noalloc(double alpha, const double* a, con
                              " bytes of scratch; the static scratch holds " + std::to_string(kNoAllocBytes) +
                              " bytes (64 MiB)");
 
-    d.a.src_off = 0;
-    d.a.dst_off = 0;
-    d.a.exp_off = 0;
-    d.a.id      = 0;
-    d.a.rows    = (int32_t) M;
-    d.a.K       = (int32_t) K;
-    d.a.rows_pad  = (int32_t) Mp;
-    d.a.K_pad     = (int32_t) Kp;
-    d.a.tile_rows = MT;
-    d.a.nr        = lc.nm;
-    d.a.nk        = lc.nk;
-    d.a.kcontig   = 1;
-    for(int j = 0; j < lc.nk; j++) d.a.kcontig &= (lc.k_a[j] == na - lc.nk + j) ? 1 : 0;
-    d.b.src_off   = 0;
-    d.b.dst_off   = abytes;
-    d.b.exp_off   = (int32_t) Mp;
-    d.b.id        = 1;
-    d.b.rows      = (int32_t) N;
-    d.b.K         = (int32_t) K;
-    d.b.rows_pad  = (int32_t) Np;
-    d.b.K_pad     = (int32_t) Kp;
-    d.b.tile_rows = NT;
-    d.b.nr        = lc.nn;
-    d.b.nk        = lc.nk;
-    d.b.kcontig   = 1;
-    for(int j = 0; j < lc.nk; j++) d.b.kcontig &= (lc.k_b[j] == nb - lc.nk + j) ? 1 : 0;
+    // the same views the allocating path builds
+    int32_t ad[kMaxModes], bd[kMaxModes];
+    for(int i = 0; i < na; i++) ad[i] = (int32_t) adims[i];
+    for(int i = 0; i < nb; i++) bd[i] = (int32_t) bdims[i];
+    d.a         = view_block(ad, na, lc.m_a, lc.nm, lc.k_a, lc.nk, MT, KC);
+    d.b         = view_block(bd, nb, lc.n_b, lc.nn, lc.k_b, lc.nk, NT, KC);
+    d.b.dst_off = abytes;
+    d.b.exp_off = (int32_t) Mp;
+    d.b.id      = 1;
     d.g.c_off      = 0;
     d.g.task_begin = 0;
     d.g.task_end   = 1;
@@ -2157,8 +1479,8 @@ extern "C" int tb_block_multiply_int8_noalloc(double alpha, const double* a, con
     d.meta.log2k  = lk;
     d.mtiles      = (int32_t) mtiles;
     d.ntiles      = (int32_t) ntiles;
-    d.nchunk_a    = (int32_t) (Mp / 8);
-    d.nchunk_b    = (int32_t) (Np / 8);
+    d.nchunk_a    = (int32_t) split_units(d.a);
+    d.nchunk_b    = (int32_t) split_units(d.b);
     d.chunks_off  = chunks_off;
 
     // set-up once per device, with that device current: the device address of the
