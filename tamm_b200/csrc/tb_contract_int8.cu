@@ -59,8 +59,13 @@ struct I8TaskMeta {
   int32_t log2k;            // ceil(log2 K) of the task
 };
 
+// One CTA's work: an output tile run whole (nparts = 1), or one segment of its K (the
+// part-th of nparts, its sums in workspace slot ws + part): nsteps K steps from step kc0 of
+// task `task` on.  `tile` numbers the tiles of the launch.
 struct I8Item {
-  int32_t group, mt, nt, pad;
+  int32_t group, mt, nt, tile;
+  int32_t task, kc0, nsteps;
+  int32_t part, nparts, ws;
 };
 
 // One output tile as the producer hands it to the MMA issuer and the epilogue through a
@@ -73,7 +78,8 @@ struct TileRec {
   int64_t c_off;
   int32_t group, mt, nt, task_begin, task_end, M, N;
   int32_t mdim[kMaxClass], mstr[kMaxClass], ndim[kMaxClass], nstr[kMaxClass];
-  int32_t pad[7];
+  int32_t kc0, nsteps, tile, part, nparts, ws; // (see I8Item)
+  int32_t pad;
 };
 static_assert(sizeof(TileRec) == 128, "tile record size");
 
@@ -128,13 +134,17 @@ struct I8Params {
   LabelClasses    lc;
   int*            err;
   const uint8_t*  tslices; // digit count of each task (1..S)
-  int*            ctr;     // next output tile to hand out (zero at launch)
+  int*            ctr;     // next item to hand out, then the split tiles' arrivals (zero at launch)
   int             xpose;   // C is contiguous along the tile's columns: transposed reductions
   int             store;   // C = alpha * result (an assignment whose output blocks this
                            // launch covers completely) instead of C += alpha * result
   int             energy = 0; // set for the EN instantiations: sum (C + alpha * result)^2 / D into en.part
   EnergyArgs      en;
+  double*         ws = nullptr; // sums of split tiles' segments, MT x NT each
 };
+// The tile counter is followed by the arrivals of split tiles, kArrive per segment (one per
+// epilogue warp, at the tile's first segment).
+constexpr int kArrive = 16;
 
 template<int S, int NT>
 __host__ __device__ constexpr uint32_t stage_bytes() {
@@ -246,8 +256,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           r.group      = item.group;
           r.mt         = item.mt;
           r.nt         = item.nt;
-          r.task_begin = g.task_begin;
+          r.task_begin = item.task;
           r.task_end   = g.task_end;
+          r.kc0        = item.kc0;
+          r.nsteps     = item.nsteps;
+          r.tile       = item.tile;
+          r.part       = item.part;
+          r.nparts     = item.nparts;
+          r.ws         = item.ws;
           int32_t cstr[kMaxModes]; // C block strides (a block holds fewer than 2^31 elements)
           int32_t sz = 1;
           for(int i = p.lc.nc - 1; i >= 0; i--) {
@@ -267,8 +283,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           }
           r.M = M;
           r.N = N;
-          if(g.task_begin < g.task_end) { // the first task's row exponents and column scales, to L1
-            const I8Task   t0 = p.tasks[g.task_begin];
+          if(item.task < g.task_end) { // the first task's row exponents and column scales, to L1
+            const I8Task   t0 = p.tasks[item.task];
             const int32_t* ea = p.a_exps + t0.a_exp + item.mt * MT;
             const int32_t* eb = p.b_exps + t0.b_exp + item.nt * NT;
 #pragma unroll
@@ -285,13 +301,15 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           qph ^= 1;
         }
         if(it >= p.nitems) break;
-        for(int t = g.task_begin; t < g.task_end; t++) {
-          const I8Task   tk = p.tasks[t];
-          const uint8_t* ga = p.a_slices + tk.a_off + (int64_t) item.mt * tk.nkc * A_BYTES;
-          const uint8_t* gb = p.b_slices + tk.b_off + (int64_t) item.nt * tk.nkc * B_BYTES;
+        for(int t = item.task, left = item.nsteps, k0 = item.kc0; t < g.task_end && left > 0; t++, k0 = 0) {
+          const I8Task   tk  = p.tasks[t];
+          const int      nkc = min(tk.nkc - k0, left); // K steps of the task that belong to the item
+          const uint8_t* ga = p.a_slices + tk.a_off + ((int64_t) item.mt * tk.nkc + k0) * A_BYTES;
+          const uint8_t* gb = p.b_slices + tk.b_off + ((int64_t) item.nt * tk.nkc + k0) * B_BYTES;
+          left -= nkc;
           const uint32_t st = p.tslices[t]; // only the task's leading digits travel
           const uint32_t ab = st * MT * 16, bb = st * NT * 16; // per K half
-          for(int kc = 0; kc < tk.nkc; kc++) {
+          for(int kc = 0; kc < nkc; kc++) {
             if(!mbar_wait(&empty[stage], phase ^ 1, p.err, 1)) goto done_producer;
             mbar_arrive_expect_tx(&full[stage], 2 * (ab + bb));
             uint8_t*       sa = smem + stage * STAGE;
@@ -326,10 +344,12 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
       while(true) {
         if(!mbar_wait(&qfull[qslot], qph, p.err, 6)) goto done_mma;
         const int it = qitem[qslot];
-        int       tb = 0, te = 0;
+        int       tb = 0, te = 0, left = 0, k0 = 0;
         if(it >= 0) {
-          tb = trec[qslot].task_begin;
-          te = trec[qslot].task_end;
+          tb   = trec[qslot].task_begin;
+          te   = trec[qslot].task_end;
+          left = trec[qslot].nsteps;
+          k0   = trec[qslot].kc0;
         }
         mbar_arrive(&qempty[qslot]);
         if(++qslot == kQueue) {
@@ -337,9 +357,10 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           qph ^= 1;
         }
         if(it < 0) break;
-        for(int t = tb; t < te; t++) {
-          const int nkc = p.tasks[t].nkc;
+        for(int t = tb; t < te && left > 0; t++, k0 = 0) {
+          const int nkc = min(p.tasks[t].nkc - k0, left);
           const int st  = p.tslices[t];
+          left -= nkc;
           for(int kc = 0; kc < nkc; kc++) {
             if(!mbar_wait(&full[stage], phase, p.err, 3)) goto done_mma;
             tc_fence_after();
@@ -443,6 +464,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
       // the slot goes back to the producer
       const TileRec& rec = trec[rslot];
       const int      imt = rec.mt, int_ = rec.nt, igroup = rec.group, tb = rec.task_begin, te = rec.task_end;
+      const int      kc0 = rec.kc0, nsteps = rec.nsteps, itile = rec.tile, part = rec.part, nparts = rec.nparts;
+      const int      iws = rec.ws;
 #pragma unroll
       for(int x = 0; x < NH; x++) racc[x] = 0.0;
       bool ok = true;
@@ -481,13 +504,14 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           }
         }
       }
-      for(int t = tb; t < te; t++, tcount++) {
+      for(int t = tb, left = nsteps, k0 = kc0; t < te && left > 0; t++, tcount++, k0 = 0) {
         // The task's metadata and column scales 2^(e_col - 7) are fetched before its
         // accumulators are complete, so their latency overlaps the task's MMAs.  The
         // scales alternate between two buffers: the readers of this buffer (two tasks
         // back) all passed the previous task's barrier below.
         const I8Task tk  = p.tasks[t];
         const int    st  = p.tslices[t];
+        left -= min(tk.nkc - k0, left);
         const int    er  = __ldg(p.a_exps + tk.a_exp + imt * MT + row);
         double*      scb = sc + (tcount & 1) * NT;
         constexpr int off = BF ? 0 : 7; // digit weights: 2^(e - 7 - 8d) (INT8), 2^e (BF16 pieces)
@@ -589,6 +613,34 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
         }
       }
       if(!ok) break;
+      if(nparts > 1) {
+        // Split tile: this segment's sums to the workspace, one slot per thread and column
+        // (full lines); of the tile's segments, the one whose warp arrives last adds this
+        // warp's piece up over all of them, in order, so the result does not depend on which
+        // one that was.  Warps need not wait for each other.
+        double* const w0   = p.ws + (int64_t) iws * (MT * NT) + et;
+        double* const w    = w0 + (int64_t) part * (MT * NT);
+        const bool    live = rowoff >= 0;
+#pragma unroll
+        for(int x = 0; x < NH; x++)
+          if(live && nof[col0 + x] >= 0) __stcg(w + x * NE, racc[x]);
+        __threadfence();
+        __syncwarp();
+        int arrived = 0;
+        if(lane == 0) arrived = atomicAdd(p.ctr + 1 + (int64_t) iws * kArrive + (warp - 2), 1);
+        if(__shfl_sync(0xffffffffu, arrived, 0) != nparts - 1) continue;
+        __threadfence();
+#pragma unroll 1
+        for(int y = 0; y < nparts; y++) {
+          const double* r = w0 + (int64_t) y * (MT * NT);
+#pragma unroll
+          for(int x = 0; x < NH; x++)
+            if(live && nof[col0 + x] >= 0) {
+              const double v = __ldcg(r + x * NE);
+              racc[x]        = y == 0 ? v : racc[x] + v;
+            }
+        }
+      }
       if constexpr(EN) {
         // sum (C + alpha * result)^2 / D over the tile; C is read, not written.  One
         // partial sum per warp and tile (each thread's elements in a fixed order, then
@@ -647,7 +699,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
         }
 #pragma unroll
         for(int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-        if(lane == 0) p.en.part[(int64_t) it * EW + (warp - 2)] = e;
+        if(lane == 0) p.en.part[(int64_t) itile * EW + (warp - 2)] = e;
         continue;
       }
       // C (+)= alpha * result: one reduction per element (c + alpha * r, rounded once,
@@ -757,7 +809,8 @@ struct I8Layout {
   int64_t                 slice_bytes = 0, a_bytes = 0;
   int64_t                 nexp = 0, a_nexp = 0;
   double                  int8_ops = 0;
-  double                  kc_per_item = 0; // mean 32-byte K steps of an output tile (all its tasks)
+  double                  kc_per_item = 0; // mean 32-byte K steps of an item
+  int64_t                 ntiles = 0, parts = 0; // output tiles; segments of those that are split
   I8Task*                 d_tasks   = nullptr;
   I8Item*                 d_items   = nullptr;
   I8TaskMeta*             d_meta    = nullptr;
@@ -793,6 +846,42 @@ void upload_vec(T*& dptr, const std::vector<T>& vec) {
   if(vec.empty()) return;
   TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&dptr), sizeof(T) * vec.size()));
   TB_CUDA(cudaMemcpy(dptr, vec.data(), sizeof(T) * vec.size(), cudaMemcpyHostToDevice));
+}
+
+// Output blocks of a few tiles with a long K (a Fock-like intermediate: 20 x 20 over K =
+// 384000 at O=40/V=160, 3.95 ms in one CTA of each spin) run as segments of kSplitSteps K
+// steps, an item each, whose sums the last of them adds up.  The rule and the cuts follow
+// the group's own admitted tasks, run or skipped, so the result depends neither on the
+// launch's other blocks nor on tasks skipped as exact zeros.  A segment takes 0.33 us per
+// step and the last one about 1 us per segment to add them up: at 256 steps both shares of
+// such a contraction are near 50-80 us.
+constexpr int64_t kSplitTiles = 8;
+constexpr int64_t kSplitSteps = 256; // in steps of 32 K elements
+
+void group_segments(const LabelClasses& lc, const WorkList& wl, int32_t group, int kstep, const I8Layout& L,
+                    std::vector<I8Item>& segs) {
+  const DevGroup& g     = wl.groups[group];
+  const int64_t   total = wl.group_chunks[group], nseg = (total + kSplitSteps - 1) / kSplitSteps;
+  if(nseg <= 1) return;
+  int64_t   seg = -1;
+  const int per = kChunkK / kstep; // steps of a 32-element chunk
+  for(int t = g.task_begin; t < g.task_end; t++) {
+    const int64_t p0 = wl.tasks[t].pos, n = task_chunks(lc, wl.tasks[t]);
+    for(int64_t c = 0; c < n;) { // the task's chunks, segment by segment
+      int64_t s = (p0 + c) * nseg / total;
+      while(total * (s + 1) / nseg <= p0 + c) s++;
+      const int64_t end = std::min(n, total * (s + 1) / nseg - p0);
+      if(s != seg) {
+        I8Item it{};
+        it.task = t;
+        it.kc0  = (int32_t) (c * per);
+        segs.push_back(it);
+        seg = s;
+      }
+      segs.back().nsteps += (int32_t) (std::min<int64_t>(end * per, L.tasks[t].nkc) - c * per);
+      c = end;
+    }
+  }
 }
 
 // ea / eb: cached digits of a read-only A / B (their blocks are not split per launch).
@@ -915,6 +1004,7 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
     mts = (M + MT - 1) / MT;
     nts = (N + L->NT - 1) / L->NT;
   };
+  std::vector<I8Item> segs;
   for(size_t r0 = 0; r0 < order.size();) {
     size_t r1 = r0 + 1; // groups [r0, r1): equal work, same first A block
     while(r1 < order.size() && order[r1].work == order[r0].work && order[r1].akey == order[r0].akey) r1++;
@@ -929,7 +1019,26 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
         int64_t gm = 0, gn = 0;
         tiles_of(order[r].group, gm, gn);
         if(mt >= gm) continue;
-        for(int64_t nt = 0; nt < gn; nt++) L->items.push_back(I8Item{order[r].group, (int32_t) mt, (int32_t) nt, 0});
+        const DevGroup& g = wl.groups[order[r].group];
+        for(int64_t nt = 0; nt < gn; nt++, L->ntiles++) {
+          I8Item it{order[r].group, (int32_t) mt, (int32_t) nt, (int32_t) L->ntiles, g.task_begin, 0, 0x7fffffff, 0, 1, 0};
+          segs.clear();
+          if(gm * gn <= kSplitTiles) group_segments(lc, wl, order[r].group, kstep, *L, segs);
+          if(segs.size() <= 1) {
+            L->items.push_back(it);
+            continue;
+          }
+          it.nparts = (int32_t) segs.size();
+          it.ws     = (int32_t) L->parts;
+          L->parts += it.nparts;
+          for(const auto& sg: segs) {
+            it.task   = sg.task;
+            it.kc0    = sg.kc0;
+            it.nsteps = sg.nsteps;
+            L->items.push_back(it);
+            it.part++;
+          }
+        }
       }
     for(size_t r = r0; r < r1; r++) {
       int64_t gm = 0, gn = 0;
@@ -959,7 +1068,8 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
   TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_tslices), std::max<size_t>(1, L->tasks.size())));
   TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_err), sizeof(int)));
   TB_CUDA(cudaMemset(L->d_err, 0, sizeof(int)));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_ctr), sizeof(int)));
+  TB_EXPECTS(L->parts * kArrive < (1ll << 30) && L->items.size() < (1ull << 31), "too many output tiles");
+  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_ctr), sizeof(int) * (1 + L->parts * kArrive)));
   return L;
 }
 
@@ -1005,7 +1115,7 @@ constexpr double kShortKSteps = 8.0;
 
 template<int S, int NT, bool BF>
 void launch_gemm(const I8Layout& L, const WorkList& wl, const LabelClasses& lc, double alpha,
-                 const uint8_t* slices, const int32_t* exps, double* C, const Plan& plan, cudaStream_t st) {
+                 const uint8_t* slices, const int32_t* exps, double* ws, double* C, const Plan& plan, cudaStream_t st) {
   if(L.items.empty()) return;
   I8Params p;
   p.a_slices = L.a_cache ? L.a_cache->slices : slices;
@@ -1029,7 +1139,8 @@ void launch_gemm(const I8Layout& L, const WorkList& wl, const LabelClasses& lc, 
     p.energy = 1;
     p.en     = *plan.energy;
   }
-  TB_CUDA(cudaMemsetAsync(L.d_ctr, 0, sizeof(int), st));
+  p.ws = ws;
+  TB_CUDA(cudaMemsetAsync(L.d_ctr, 0, sizeof(int) * (1 + L.parts * kArrive), st));
   const size_t smem = smem_bytes<S, NT>();
   static bool  configured[64][3] = {};
   int          dev            = 0;
@@ -1057,22 +1168,22 @@ void launch_gemm(const I8Layout& L, const WorkList& wl, const LabelClasses& lc, 
   else k_contract_i8<S, NT, BF><<<grid, NTHREADS, smem, st>>>(p);
   TB_CUDA(cudaGetLastError());
   if(plan.energy)
-    launch_energy_final(p.en.part, (int64_t) L.items.size() * (NEPI / 32), plan.energy_scale, plan.energy_out, st);
+    launch_energy_final(p.en.part, L.ntiles * (NEPI / 32), plan.energy_scale, plan.energy_out, st);
 }
 
 template<int S, bool BF = false>
 void run_s(const I8Layout& L, const WorkList& wl, const LabelClasses& lc, double alpha, const double* A,
-           const double* B, double* C, uint8_t* slices, int32_t* exps, const Plan& plan, cudaStream_t st,
+           const double* B, double* C, uint8_t* slices, int32_t* exps, double* ws, const Plan& plan, cudaStream_t st,
            cudaEvent_t* ev) {
   if(ev) TB_CUDA(cudaEventRecord(ev[0], st));
   launch_split<S, BF>(L, wl, A, B, slices, exps, st);
   if(ev) TB_CUDA(cudaEventRecord(ev[1], st));
   // output tile width: 80 columns by default for S <= 6 (S x NT <= 512 TMEM columns)
   if constexpr(S * 80 <= 512) {
-    if(L.NT == 80) launch_gemm<S, 80, BF>(L, wl, lc, alpha, slices, exps, C, plan, st);
+    if(L.NT == 80) launch_gemm<S, 80, BF>(L, wl, lc, alpha, slices, exps, ws, C, plan, st);
   }
-  if(L.NT == 64) launch_gemm<S, 64, BF>(L, wl, lc, alpha, slices, exps, C, plan, st);
-  if(L.NT == 48) launch_gemm<S, 48, BF>(L, wl, lc, alpha, slices, exps, C, plan, st);
+  if(L.NT == 64) launch_gemm<S, 64, BF>(L, wl, lc, alpha, slices, exps, ws, C, plan, st);
+  if(L.NT == 48) launch_gemm<S, 48, BF>(L, wl, lc, alpha, slices, exps, ws, C, plan, st);
   if(ev) TB_CUDA(cudaEventRecord(ev[2], st));
 }
 
@@ -1183,6 +1294,8 @@ void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* 
   const int64_t ebytes = sizeof(int32_t) * std::max<int64_t>(L->nexp, 1);
   auto* slices = static_cast<uint8_t*>(plan.pinned ? plan.pinned->get(L->slice_bytes) : sc.get(L->slice_bytes));
   auto* exps   = static_cast<int32_t*>(plan.pinned ? plan.pinned->get(ebytes) : sc.get(ebytes));
+  const int64_t wbytes = 8 * L->parts * MT * NT; // split tiles' sums
+  auto* ws = wbytes == 0 ? nullptr : static_cast<double*>(plan.pinned ? plan.pinned->get(wbytes) : sc.get(wbytes));
   cudaEvent_t  evs[3];
   cudaEvent_t* ev = nullptr;
   if(plan.profile) {
@@ -1190,20 +1303,22 @@ void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* 
     ev = evs;
   }
   const Plan& st = plan;
-  if(bf) run_s<2, true>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev);
+  if(bf) run_s<2, true>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev);
   else switch(S) {
-    case 3: run_s<3>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
-    case 4: run_s<4>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
-    case 5: run_s<5>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
-    case 6: run_s<6>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
-    case 7: run_s<7>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
-    default: run_s<8>(*L, wl, lc, alpha, A, B, C, slices, exps, st, stream, ev); break;
+    case 3: run_s<3>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
+    case 4: run_s<4>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
+    case 5: run_s<5>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
+    case 6: run_s<6>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
+    case 7: run_s<7>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
+    default: run_s<8>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
   }
   if(plan.pinned) {
+    if(ws) plan.pinned->put(ws);
     plan.pinned->put(exps);
     plan.pinned->put(slices);
   }
   else {
+    if(ws) sc.put(ws);
     sc.put(exps);
     sc.put(slices);
   }
@@ -1227,6 +1342,7 @@ void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* 
     double ops = 0, alg = 0;
     int    smin = S, smax = 1;
     for(const auto& it: L->items) {
+      if(it.part > 0) continue; // (per tile, all its tasks)
       const DevGroup& g = wl.groups[it.group];
       int64_t         M = 1, N = 1;
       for(int j = 0; j < lc.nm; j++) M *= g.cdims[lc.m_c[j]];
@@ -1345,7 +1461,7 @@ __global__ void k_noalloc_setup(NoAllocDesc d, unsigned char* base) {
       d.meta;
   }
   I8Item* items = reinterpret_cast<I8Item*>(base + kCtlItems);
-  for(int i = tid; i < d.mtiles * d.ntiles; i += nth) items[i] = I8Item{0, i / d.ntiles, i % d.ntiles, 0};
+  for(int i = tid; i < d.mtiles * d.ntiles; i += nth) items[i] = I8Item{0, i / d.ntiles, i % d.ntiles, i, 0, 0, 0x7fffffff, 0, 1, 0};
   if(tid == 0) { // one block per operand: first unit 0, then the unit count
     int32_t* cb = reinterpret_cast<int32_t*>(base + d.chunks_off);
     cb[0] = 0, cb[1] = d.nchunk_a, cb[2] = 0, cb[3] = d.nchunk_b;
@@ -1445,7 +1561,7 @@ extern "C" int tb_block_multiply_int8_noalloc(double alpha, const double* a, con
     const int64_t Mp = rup(M, MT), Np = rup(N, NT), Kp = rup(K, KC);
     const int64_t abytes = S * Mp * Kp, bbytes = S * Np * Kp;
     const int64_t mtiles = Mp / MT, ntiles = Np / NT;
-    const int64_t chunks_off = rup(kCtlItems + 16 * mtiles * ntiles, 256);
+    const int64_t chunks_off = rup(kCtlItems + (int64_t) sizeof(I8Item) * mtiles * ntiles, 256);
     const int64_t exps_off   = rup(chunks_off + 16, 256);
     const int64_t sl_off     = rup(exps_off + 4 * (Mp + Np), 256);
     const int64_t need       = sl_off + abytes + bbytes;
