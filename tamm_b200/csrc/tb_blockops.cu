@@ -648,6 +648,277 @@ void launch_assign_blocks(double* dst, double scale, const double* src, const Bl
   TB_CUDA(cudaGetLastError());
 }
 
+bool make_fused_block(const AssignLoop* loops, const int64_t* src_off, int present, int n, int64_t dst_off,
+                      int64_t units, FusedBlock& b) {
+  b         = FusedBlock{};
+  b.dst_off = dst_off;
+  b.first   = units;
+  b.present = present;
+  const AssignLoop* l0 = nullptr;
+  for(int k = 0; k < n; k++)
+    if(present >> k & 1) l0 = l0 ? l0 : &loops[k];
+  if(l0 == nullptr || l0->nd < 2) return false;
+  const int nd = l0->nd, q = nd - 1;
+  b.nd = nd;
+  b.p  = -1;
+  int64_t total = 1, dsize = 1;
+  for(int d = 0; d < nd; d++) {
+    total *= l0->dims[d];
+    dsize += (l0->dims[d] - 1) * l0->dld[d];
+  }
+  if(total <= 0 || total >= (int64_t(1) << 31) || dsize >= (int64_t(1) << 31) || (l0->dims[q] > 1 && l0->dld[q] != 1))
+    return false;
+  for(int k = 0; k < n; k++) {
+    if(!(present >> k & 1)) continue;
+    const AssignLoop& l = loops[k];
+    int64_t           ssize = 1;
+    for(int d = 0; d < nd; d++) {
+      if(l.dims[d] != l0->dims[d] || l.dld[d] != l0->dld[d]) return false;
+      ssize += (l.dims[d] - 1) * l.sld[d];
+    }
+    if(ssize >= (int64_t(1) << 31)) return false;
+    b.src_off[k] = src_off[k];
+    for(int d = 0; d < nd; d++) b.sld[k][d] = (int32_t) l.sld[d];
+    if(l.sld[q] == 1 || l.dims[q] == 1) continue; // rows along q on both sides
+    int p = -1;
+    for(int d = 0; d < q; d++)
+      if(l.sld[d] == 1 && l.dims[d] > 1) p = d;
+    if(p < 0 || (b.p >= 0 && b.p != p)) return false;
+    b.p = p;
+    b.staged |= 1 << k;
+  }
+  if(b.p < 0) b.p = nd - 2;
+  int64_t outer = 1;
+  for(int d = 0; d < 4; d++) {
+    b.dims[d] = (int32_t) (d < nd ? l0->dims[d] : 1);
+    b.dld[d]  = (int32_t) (d < nd ? l0->dld[d] : 0);
+    b.mag[d]  = asg_magic64(b.dims[d]);
+    if(d < nd && d != b.p && d != q) outer *= l0->dims[d];
+  }
+  const int64_t nbq = (b.dims[q] + kAsgQ - 1) / kAsgQ, nbp = (b.dims[b.p] + kAsgP - 1) / kAsgP;
+  const int64_t tq = (b.dims[q] + nbq - 1) / nbq, tp = (b.dims[b.p] + nbp - 1) / nbp;
+  b.nbq      = (int32_t) nbq;
+  b.nbp      = (int32_t) nbp;
+  b.tq       = (int32_t) tq;
+  b.tp       = (int32_t) tp;
+  b.nsub     = (int32_t) (outer * nbq * nbp);
+  b.per_unit = (int32_t) std::max<int64_t>(
+    1, std::min<int64_t>({(int64_t) kAsgMaxSub, kAsgN / (tq * tp), kAsgStage / (tq * (tp | 1))}));
+  b.units  = (b.nsub + b.per_unit - 1) / b.per_unit;
+  b.mag[4] = asg_magic64(nbq);
+  b.mag[5] = asg_magic64(nbp);
+  return units + b.units < (int64_t(1) << 31);
+}
+
+namespace {
+
+// Records of a fused unit: origins of its sub-tiles in the destination and in every op's
+// source, and their extents (nq | np << 16).
+struct FusedUnit {
+  int dof[kAsgMaxSub], ext[kAsgMaxSub];
+  int so[kFuseOps][kAsgMaxSub];
+};
+
+__device__ __forceinline__ void fused_records(const FusedBlock& a, int lu, FusedUnit& r) {
+  const int t = threadIdx.x, q = a.nd - 1, p = a.p, t0 = lu * a.per_unit;
+  if(t >= a.per_unit || t0 + t >= a.nsub) return;
+  int       x  = t0 + t;
+  int       y  = asg_div64(x, a.mag[4]);
+  const int bq = x - y * a.nbq;
+  x            = asg_div64(y, a.mag[5]);
+  const int bp = y - x * a.nbp;
+  const int q0 = bq * a.tq, p0 = bp * a.tp;
+  int       doff = q0 * a.dld[q] + p0 * a.dld[p], so[kFuseOps];
+#pragma unroll
+  for(int k = 0; k < kFuseOps; k++) so[k] = q0 * a.sld[k][q] + p0 * a.sld[k][p];
+  for(int d = a.nd - 1; d >= 0; d--) {
+    if(d == q || d == p) continue;
+    const int z = asg_div64(x, a.mag[d]), i = x - z * a.dims[d];
+    x           = z;
+    doff += i * a.dld[d];
+#pragma unroll
+    for(int k = 0; k < kFuseOps; k++) so[k] += i * a.sld[k][d];
+  }
+  r.dof[t] = doff;
+  r.ext[t] = min(a.tq, a.dims[q] - q0) | (min(a.tp, a.dims[p] - p0) << 16);
+#pragma unroll
+  for(int k = 0; k < kFuseOps; k++) r.so[k][t] = so[k];
+}
+
+// The staged ops' elements of a unit, row by row along p (odd row pitch), an op's tile
+// after the other.  A thread keeps its places within the sub-tile over the unit's sub-tiles.
+__device__ __forceinline__ void fused_load(const FusedBlock& a, int lu, const FusedUnit& r,
+                                           const double* __restrict__ src, uint32_t stage) {
+  const int staged = a.staged;
+  if(staged == 0) return;
+  const int TQ = a.tq, TP = a.tp, pitch = TP | 1, ns = min(a.per_unit, a.nsub - lu * a.per_unit);
+  const int qd = a.nd - 1;
+  int       left = staged;
+  for(int n = 0; left; n++, left &= left - 1) {
+    const int      k  = __ffs(left) - 1, sq = a.sld[k][qd];
+    const double*  s0 = src + a.src_off[k];
+    const int*     so = r.so[k];
+    const unsigned mp = asg_magic(TP);
+    for(int e = threadIdx.x; e < TQ * TP; e += kThreads) {
+      const int      iq = asg_div(e, mp), ip = e - iq * TP;
+      const double*  se = s0 + iq * sq + ip;
+      const uint32_t to = stage + (uint32_t) (n * kAsgStage + iq * pitch + ip) * 8u;
+#pragma unroll 4
+      for(int t = 0; t < ns; t++) {
+        const int ext = r.ext[t];
+        if(iq < (ext & 0xFFFF) && ip < (ext >> 16))
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(to + (uint32_t) (t * TQ * pitch) * 8u),
+                       "l"(se + so[t]));
+      }
+    }
+  }
+}
+
+} // namespace
+
+// A run of AddOps in one pass: each element's old value, then the ops' terms in op order
+// with the ops' own roundings, so the result equals the separate passes bit for bit.  Bound
+// by HBM (the destination and the source once each); the separate passes read the source
+// and read and write the destination once per op.  Neighbouring units go to CTAs running at
+// the same time, and the host lists blocks that share their source blocks one after the
+// other, so that the other ops' reads of a source block come from L2.  What it reaches is
+// set by the units' latency and instructions (a unit is up to 2048 elements between two
+// barriers): small units on four CTAs per SM, no pipeline within a CTA (with a second stage
+// and two CTAs 930 us).  The four adds of P(ab) P(ij) on an r2 of 0.62 GB: 718 us, 1430 in
+// four passes; 192 would be the bytes alone.
+__global__ void __launch_bounds__(kThreads, 4) k_fused_adds(double* __restrict__ dst, const double* __restrict__ src,
+                                                            const FusedBlock* __restrict__ blocks, int nblocks,
+                                                            int nunits, FusedOps ops) {
+  extern __shared__ __align__(16) double fsm[]; // a tile of kAsgStage doubles per staged op
+  __shared__ FusedUnit                   recs[2];
+  __shared__ int                         s_pair;
+  const int G = gridDim.x, u0 = blockIdx.x;
+  if(u0 >= nunits) return;
+  if(threadIdx.x == 0) { // the block holding unit u0: last one with first <= u0
+    int lo = 0, hi = nblocks - 1;
+    while(lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if(blocks[mid].first <= u0) lo = mid;
+      else hi = mid - 1;
+    }
+    s_pair = lo;
+  }
+  __syncthreads();
+  auto block_of = [&](int pi, int u) {
+    while(u >= blocks[pi].first + blocks[pi].units) pi++;
+    return pi;
+  };
+  int pi = block_of(s_pair, u0), slot = 0;
+  fused_records(blocks[pi], u0 - (int) blocks[pi].first, recs[0]);
+  __syncthreads();
+  for(int u = u0; u < nunits; u += G, slot ^= 1) {
+    const FusedBlock& a   = blocks[pi];
+    const FusedUnit&  rec = recs[slot];
+    const int         lu  = u - (int) a.first;
+    fused_load(a, lu, rec, src, (uint32_t) __cvta_generic_to_shared(fsm));
+    if(u + G < nunits) { // the next unit's records while the copies are on their way
+      pi = block_of(pi, u + G);
+      fused_records(blocks[pi], u + G - (int) blocks[pi].first, recs[slot ^ 1]);
+    }
+    const int         TQ = a.tq, pitch = a.tp | 1, dp = a.dld[a.p], ns = min(a.per_unit, a.nsub - lu * a.per_unit);
+    double* const     d0 = dst + a.dst_off;
+    const int         present = a.present, staged = a.staged;
+    const bool        keep = !(ops.assign && (present & 1)); // the old values count
+    const double*     s0[kFuseOps];
+    int               sp[kFuseOps], tl[kFuseOps]; // source, its stride along p, or the op's tile
+#pragma unroll
+    for(int k = 0, n = 0; k < kFuseOps; k++) {
+      s0[k] = src + a.src_off[k];
+      sp[k] = a.sld[k][a.p];
+      tl[k] = n * kAsgStage;
+      n += staged >> k & 1;
+    }
+    if(staged) { // this thread's copies have landed, and every other thread's
+      asm volatile("cp.async.wait_all;\n" ::: "memory");
+      __syncthreads();
+    }
+    // A thread keeps its places (ip, iq) within the sub-tile, consecutive threads along q, over
+    // the unit's sub-tiles; X sub-tiles' loads in flight together.
+    constexpr int  X  = 2;
+    const unsigned mq = asg_magic(TQ);
+    for(int e = threadIdx.x; e < TQ * a.tp; e += kThreads) {
+      const int ip = asg_div(e, mq), c = e - ip * TQ;
+      double*   d  = d0 + ip * dp + c;
+      const double* se[kFuseOps]; // this place's element of a sub-tile at origin 0, in memory or in the op's tile
+#pragma unroll
+      for(int k = 0; k < kFuseOps; k++) se[k] = staged >> k & 1 ? fsm + tl[k] + c * pitch + ip : s0[k] + ip * sp[k] + c;
+      for(int t0 = 0; t0 < ns; t0 += X) {
+        double v[X], x[kFuseOps][X];
+        int    at[X];
+        bool   on[X];
+#pragma unroll
+        for(int y = 0; y < X; y++) {
+          const int t = min(t0 + y, ns - 1), ext = rec.ext[t];
+          at[y]       = rec.dof[t];
+          on[y]       = t0 + y < ns && c < (ext & 0xFFFF) && ip < (ext >> 16);
+          v[y]        = 0.0;
+        }
+        if(keep) {
+#pragma unroll
+          for(int y = 0; y < X; y++)
+            if(on[y]) v[y] = d[at[y]];
+        }
+#pragma unroll
+        for(int k = 0; k < kFuseOps; k++) {
+          if(staged >> k & 1) {
+#pragma unroll
+            for(int y = 0; y < X; y++) x[k][y] = se[k][min(t0 + y, ns - 1) * TQ * pitch];
+          }
+          else if(present >> k & 1) {
+#pragma unroll
+            for(int y = 0; y < X; y++) x[k][y] = on[y] ? __ldg(se[k] + rec.so[k][min(t0 + y, ns - 1)]) : 0.0;
+          }
+        }
+#pragma unroll
+        for(int k = 0; k < kFuseOps; k++) {
+          const double al = ops.alpha[k];
+          if(!(present >> k & 1)) continue;
+          if(k == 0 && !keep) {
+#pragma unroll
+            for(int y = 0; y < X; y++) v[y] = __dmul_rn(al, x[k][y]);
+          }
+          else if(ops.flat >> k & 1) {
+#pragma unroll
+            for(int y = 0; y < X; y++) v[y] = fma(al, x[k][y], v[y]);
+          }
+          else {
+#pragma unroll
+            for(int y = 0; y < X; y++) v[y] = __dadd_rn(v[y], __dmul_rn(al, x[k][y]));
+          }
+        }
+#pragma unroll
+        for(int y = 0; y < X; y++)
+          if(on[y]) d[at[y]] = v[y];
+      }
+    }
+    __syncthreads(); // the tiles and this unit's records are free, the next unit's complete
+  }
+}
+
+void launch_fused_adds(double* dst, const double* src, const FusedBlock* blocks, int nblocks, int64_t nunits,
+                       int staged, const FusedOps& ops, cudaStream_t stream) {
+  if(nblocks <= 0 || nunits <= 0) return;
+  TB_EXPECTS(nunits < (int64_t(1) << 31), "too many work units in one add");
+  const int   smem            = staged * kAsgStage * 8;
+  static bool configured[64] = {false};
+  int         dev = 0, nsm = 0, per_sm = 0;
+  TB_CUDA(cudaGetDevice(&dev));
+  if(dev < 64 && !configured[dev]) {
+    TB_CUDA(cudaFuncSetAttribute(k_fused_adds, cudaFuncAttributeMaxDynamicSharedMemorySize, kFuseOps * kAsgStage * 8));
+    configured[dev] = true;
+  }
+  TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_fused_adds, kThreads, smem));
+  TB_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int64_t grid = std::min<int64_t>(nunits, (int64_t) nsm * std::max(per_sm, 1));
+  k_fused_adds<<<(unsigned) grid, kThreads, smem, stream>>>(dst, src, blocks, nblocks, (int) nunits, ops);
+  TB_CUDA(cudaGetLastError());
+}
+
 void launch_fill(double* x, int64_t n, double value, int is_assign, cudaStream_t stream) {
   if(n <= 0) return;
   k_fill<<<grid_for(n, 8), kThreads, 0, stream>>>(x, n, value, is_assign);

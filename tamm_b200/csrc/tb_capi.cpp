@@ -1396,6 +1396,7 @@ int tb_sched_release(tb_sched s) {
   s->p->plan_cache.clear();
   s->p->wl_cache.clear();
   s->p->fill_cache.clear();
+  s->p->fuse_cache.clear();
   TB_API_END
 }
 

@@ -259,6 +259,33 @@ BlockAssign make_block_assign(const AssignLoop& lp, int64_t dst_off, int64_t src
 // holding nunits work units in all).
 void launch_assign_blocks(double* dst, double scale, const double* src, const BlockAssign* blocks, int nblocks,
                           int64_t nunits, int is_assign, cudaStream_t stream);
+// Consecutive AddOps dst (=|+=) alpha_k * src(permuted labels) of one destination and one
+// source, run in one pass: the destination's blocks, each with the source block and strides
+// of every op that applies to it (`present`; `staged`: through the shared-memory transpose,
+// whose plane's other mode is `p` for all of them).  Units as in BlockAssign, always
+// sub-tiles of the (q, p) plane.
+constexpr int kFuseOps = 4;
+struct FusedBlock {
+  int64_t  dst_off, first;
+  int32_t  nd, p;
+  int32_t  dims[4], dld[4];
+  int32_t  units, per_unit, tq, tp, nsub, nbq, nbp;
+  int32_t  present, staged;
+  int64_t  src_off[kFuseOps];
+  int32_t  sld[kFuseOps][4];
+  uint64_t mag[6]; // multipliers for dims[0..3], nbq, nbp
+};
+struct FusedOps {
+  int32_t n, assign;       // ops; the first one assigns
+  int32_t flat;            // ops of equal layout (bit per op): one fused multiply-add, as the flat add
+  double  alpha[kFuseOps];
+};
+// False where the ops cannot share a pass over this block (more than one transposing mode,
+// 2^31 elements and more); `units` counts the launch's work units.
+bool make_fused_block(const AssignLoop* loops, const int64_t* src_off, int present, int n, int64_t dst_off,
+                      int64_t units, FusedBlock& out);
+void launch_fused_adds(double* dst, const double* src, const FusedBlock* blocks, int nblocks, int64_t nunits,
+                       int staged, const FusedOps& ops, cudaStream_t stream);
 void launch_fill(double* x, int64_t n, double value, int is_assign, cudaStream_t stream);
 // Segment lists of the block-wise fill and map: per run of blocks (dst offset, src
 // offset or -1, n, first), `first` the sum of n over the runs before it.

@@ -512,6 +512,17 @@ bool same_target(const Labeled& x, const Labeled& y) {
   return true;
 }
 
+// FlatAddPlan condition (addop.hpp:245-251): same labels, same layout
+bool flat_add(const Op& op) {
+  bool flat = op.lhs.labels == op.a.labels && op.lhs.t->has_spin == op.a.t->has_spin &&
+              op.lhs.t->nmodes == op.a.t->nmodes && op.lhs.t->keys == op.a.t->keys &&
+              op.lhs.t->offsets == op.a.t->offsets;
+  for(int i = 0; flat && i < op.lhs.t->nmodes; i++)
+    flat = op.lhs.ltis[i]->tiles == op.lhs.t->tis[i]->tiles && op.a.ltis[i]->tiles == op.a.t->tis[i]->tiles &&
+           op.lhs.t->tis[i]->tiles == op.a.t->tis[i]->tiles && op.lhs.t->tis[i]->root == op.a.t->tis[i]->root;
+  return flat;
+}
+
 std::string signature(const Op& op) {
   std::ostringstream os;
   auto               put = [&](const Labeled& x) {
@@ -804,18 +815,16 @@ void Sched::run(Op& op) {
   if(op.kind == Op::Add) {
     op.lhs.t->require_allocated();
     op.a.t->require_allocated();
+    if(op.fused_done) return;
+    if(op.fused) {
+      launch_fused_adds(op.lhs.t->data, op.a.t->data, op.fused->d, op.fused->nblocks, op.fused->units, op.fused->staged,
+                        op.fused_ops, st);
+      return;
+    }
     if(!op.add_blocks) {
       auto blocks = std::make_shared<std::vector<Op::AddBlock>>();
-      // FlatAddPlan condition (addop.hpp:245-251): same labels, same layout
-      bool flat = op.lhs.labels == op.a.labels && op.lhs.t->has_spin == op.a.t->has_spin &&
-                  op.lhs.t->nmodes == op.a.t->nmodes && op.lhs.t->keys == op.a.t->keys &&
-                  op.lhs.t->offsets == op.a.t->offsets;
-      for(int i = 0; flat && i < op.lhs.t->nmodes; i++)
-        flat = op.lhs.ltis[i]->tiles == op.lhs.t->tis[i]->tiles &&
-               op.a.ltis[i]->tiles == op.a.t->tis[i]->tiles &&
-               op.lhs.t->tis[i]->tiles == op.a.t->tis[i]->tiles &&
-               op.lhs.t->tis[i]->root == op.a.t->tis[i]->root;
-      op.flat = flat;
+      const bool flat = flat_add(op);
+      op.flat         = flat;
       if(!flat) {
         // LHSAddPlan (addop.hpp:457-519): loop over the merged labels, skip pairs with
         // a non-admitted side, apply the block assign.
@@ -1019,6 +1028,122 @@ void Sched::prepare_mult(Op& op) {
   }
   op.plan = pit->second;
   op.wl   = wl_cache[sig];
+}
+
+FusedList::~FusedList() {
+  if(!d) return;
+  int cur = -1;
+  cudaGetDevice(&cur);
+  cudaSetDevice(device);
+  cudaFree(d);
+  if(cur >= 0) cudaSetDevice(cur);
+}
+
+// A run of two to four Adds from ops[first] on that share their destination (tensor and
+// labels) and their source tensor, each with the destination's labels in some order - the
+// four terms of P(ab) P(ij), say - goes through one kernel: the destination is read and
+// written once instead of once per op.  Only the first may assign.  Their blocks are those
+// the separate ops would visit (LHSAddPlan: both sides admitted), op by op.
+void Sched::fuse_adds(size_t first) {
+  Op&       head = ops[first];
+  const int nd   = head.lhs.t ? head.lhs.t->nmodes : 0;
+  auto      fits = [&](const Op& op, bool is_head) {
+    if(op.kind != Op::Add || op.fused_done || op.add_blocks || (!is_head && op.is_assign) || op.a.t != head.a.t ||
+       op.a.t == op.lhs.t || op.a.t->is_lambda() || op.a.t->nmodes != nd || !same_target(op.lhs, head.lhs))
+      return false;
+    std::vector<bool> taken(nd, false);
+    for(int i = 0; i < nd; i++) {
+      const int p = find_label(op.lhs.labels, op.a.labels[i]);
+      if(p < 0 || taken[p] || op.a.ltis[i]->root != op.lhs.ltis[p]->root || op.a.ltis[i]->tiles != op.lhs.ltis[p]->tiles)
+        return false;
+      taken[p] = true;
+    }
+    return true;
+  };
+  if(nd < 2 || nd > 4 || head.lhs.t->is_lambda() || !fits(head, true)) return;
+  std::set<int> unique(head.lhs.labels.begin(), head.lhs.labels.end());
+  if((int) unique.size() != nd) return;
+  size_t n = 1;
+  while(n < kFuseOps && first + n < ops.size() && fits(ops[first + n], false)) n++;
+  if(n < 2) return;
+  std::string key = "U";
+  for(size_t k = 0; k < n; k++) key += "|" + std::to_string(ops[first + k].is_assign) + signature(ops[first + k]);
+  auto& list = fuse_cache[key];
+  if(!list) {
+    list         = std::make_shared<FusedList>();
+    list->device = ctx->device;
+    list->fits   = true;
+    try {
+      struct Entry {
+        int64_t                 key, dst;
+        int                     present = 0;
+        std::vector<AssignLoop> loops;
+        int64_t                 src[kFuseOps] = {0, 0, 0, 0};
+      };
+      std::vector<Entry>                             entries;
+      const auto                                     lm = tile_maps(head.lhs);
+      std::vector<std::vector<std::vector<int64_t>>> rm;
+      for(size_t k = 0; k < n; k++) rm.push_back(tile_maps(ops[first + k].a));
+      std::vector<int64_t> nt, it(nd, 0), lid(nd), rid(nd), ddims(nd), sdims(nd);
+      bool                 empty = false;
+      for(int i = 0; i < nd; i++) nt.push_back(head.lhs.ltis[i]->ntiles());
+      for(auto x: nt) empty |= x == 0;
+      if(!empty) do {
+          for(int i = 0; i < nd; i++) lid[i] = lm[i][it[i]];
+          if(!head.lhs.t->is_non_zero(lid.data())) continue;
+          Entry e;
+          e.dst = head.lhs.t->locate(lid.data());
+          e.key = INT64_MAX;
+          e.loops.resize(n);
+          for(int i = 0; i < nd; i++) ddims[i] = head.lhs.t->tis[i]->size(lid[i]);
+          for(size_t k = 0; k < n; k++) {
+            const Labeled& a = ops[first + k].a;
+            for(int i = 0; i < nd; i++) {
+              rid[i]   = rm[k][i][it[find_label(head.lhs.labels, a.labels[i])]];
+              sdims[i] = a.t->tis[i]->size(rid[i]);
+            }
+            if(!a.t->is_non_zero(rid.data())) continue;
+            e.present |= 1 << k;
+            e.src[k]   = a.t->locate(rid.data());
+            e.key      = std::min(e.key, e.src[k]);
+            e.loops[k] = plan_assign(ddims.data(), head.lhs.labels.data(), nd, sdims.data(), a.labels.data(), nd);
+          }
+          if(e.present) entries.push_back(std::move(e));
+        } while(next_tuple(it, nt));
+      // blocks with the same lowest source block share their sources: one after the other
+      std::stable_sort(entries.begin(), entries.end(), [](const Entry& a, const Entry& b) { return a.key < b.key; });
+      std::vector<FusedBlock> blocks;
+      for(const auto& e: entries) {
+        FusedBlock b;
+        if(!make_fused_block(e.loops.data(), e.src, e.present, (int) n, e.dst, list->units, b)) {
+          list->fits = false;
+          break;
+        }
+        list->units += b.units;
+        list->staged = std::max(list->staged, __builtin_popcount((unsigned) b.staged));
+        blocks.push_back(b);
+      }
+      if(blocks.size() >= (1u << 31)) list->fits = false;
+      if(list->fits && !blocks.empty()) {
+        TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&list->d), sizeof(FusedBlock) * blocks.size()));
+        TB_CUDA(cudaMemcpy(list->d, blocks.data(), sizeof(FusedBlock) * blocks.size(), cudaMemcpyHostToDevice));
+        list->nblocks = (int) blocks.size();
+      }
+    } catch(const Error&) { // an op that cannot run: reported by the op itself, in its turn
+      list->fits = false;
+    }
+  }
+  if(!list->fits) return;
+  FusedOps f{};
+  f.n      = (int) n;
+  f.assign = head.is_assign;
+  for(size_t k = 0; k < n; k++) {
+    f.alpha[k] = ops[first + k].alpha;
+    f.flat |= (flat_add(ops[first + k]) ? 1 : 0) << k;
+    ops[first + k].fused_done = k > 0;
+  }
+  head.fused     = list;
+  head.fused_ops = f;
 }
 
 // Assignment C = alpha * A * B, queued as Set(0) + Mult (MultOp::canonicalize,
@@ -1453,6 +1578,7 @@ void Sched::execute(bool profile) {
        ops[i + 1].a.t != ops[i].lhs.t && ops[i + 1].b.t != ops[i].lhs.t && // C read as an operand needs the fill
        !ops[i + 1].a.t->is_lambda() && !ops[i + 1].b.t->is_lambda())      // (a batched op adds batch by batch)
       fuse_assign(ops[i], ops[i + 1]);
+    if(!profile && ops[i].kind == Op::Add) fuse_adds(i); // (a profile times the ops one by one)
     run(ops[i]);
     note_zeros(ops[i], szero);
     if(ops[i].kind == Op::Mult && deferred_checks && ops[i].wl) pending.push_back(ops[i].wl);

@@ -213,6 +213,10 @@ struct Op {
   std::shared_ptr<int64_t>               add_dev;   // device BlockAssign list (scheduler's cache)
   int                                    add_n = 0;
   int64_t                                add_units = 0; // work units of the list
+  // a run of Adds executed in one pass: the list on its first op, the others are done with it
+  std::shared_ptr<struct FusedList>      fused;
+  FusedOps                               fused_ops{};
+  bool                                   fused_done = false;
   int                                    fn = 0;     // Map: element function
   std::shared_ptr<int64_t>               map_dev;    // Map: device segment list (seg_list)
   int                                    map_n = 0;  // runs in the list
@@ -232,6 +236,15 @@ struct Op {
   // execute (one byte per stored block; null: nothing known): an earlier assignment of
   // the same op list left them without any contribution
   std::shared_ptr<const std::vector<uint8_t>> za, zb;
+};
+
+// Device list of a run of Adds that share one pass (none: nblocks 0 and fits false).
+struct FusedList {
+  FusedBlock* d       = nullptr;
+  int         nblocks = 0, staged = 0, device = 0;
+  int64_t     units   = 0;
+  bool        fits    = false;
+  ~FusedList();
 };
 
 // Orbital energies over a root index space (device copy) and per-mode signs of a
@@ -284,6 +297,7 @@ struct Sched {
   // device block lists of SetOps over some of a tensor's blocks, by the op's signature
   // (or, for the fill of a fused assignment, its contraction's), uploaded once
   std::map<std::string, std::shared_ptr<int64_t>>  fill_cache;
+  std::map<std::string, std::shared_ptr<FusedList>> fuse_cache; // runs of Adds, by their ops' signatures
   std::map<std::string, int>                        map_count; // triples of each cached map list
   std::map<std::string, int64_t>                    add_units; // work units of each cached add list
   std::map<std::string, int64_t>                    seg_total; // elements of each cached segment list
@@ -313,6 +327,7 @@ struct Sched {
   void                                              prepare_mult(Op& op);
   void note_zeros(const Op& op, std::map<const Tensor*, std::shared_ptr<std::vector<uint8_t>>>& szero);
   void                                              fuse_assign(Op& set, Op& mult);
+  void                                              fuse_adds(size_t first);
   void                                              tune(Op& op, const std::string& key);
   double*                                           scalars();
   ~Sched();
