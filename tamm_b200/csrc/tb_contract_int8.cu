@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
               const int64_t ro = __shfl_sync(0xffffffffu, rowoff, r);
               if(ro >= 0 && o >= 0) {
                 if(p.store) p.C[ro + o] = xb[csub * kXStride + r];
-                else atomicAdd(p.C + ro + o, xb[csub * kXStride + r]);
+                else red_add(p.C + ro + o, xb[csub * kXStride + r]);
               }
             }
             __syncwarp(); // the next columns overwrite the buffer
@@ -741,7 +741,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           const int o = nof[col0 + x];
           if(o >= 0) {
             if(p.store) crow[o] = p.alpha * racc[x];
-            else atomicAdd(crow + o, p.alpha * racc[x]);
+            else red_add(crow + o, p.alpha * racc[x]);
           }
         }
       }
