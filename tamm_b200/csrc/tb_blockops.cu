@@ -2,6 +2,7 @@
 // axpby (flat AddOp / the bufacc axpy), deterministic dot / norm reductions, and the
 // seeded counter-based generator.
 #include "tb_internal.hpp"
+#include "tb_runtime.hpp"
 
 #include <algorithm>
 #include <cmath>
@@ -1119,13 +1120,14 @@ void launch_axpby(double alpha, const double* x, double beta, double* y, int64_t
 
 double reduce_dot(const double* x, const double* y, int64_t n, cudaStream_t stream) {
   if(n <= 0) return 0.0;
-  double* part = nullptr;
-  TB_CUDA(cudaMallocAsync(reinterpret_cast<void**>(&part), sizeof(double) * (kRedBlocks + 1), stream));
+  Scratch sc; // (from the kept pool)
+  sc.stream    = stream;
+  double* part = static_cast<double*>(sc.get(sizeof(double) * (kRedBlocks + 1)));
   k_dot_partial<<<kRedBlocks, kThreads, 0, stream>>>(x, y, n, part);
   k_dot_final<<<1, 1024, 0, stream>>>(part, kRedBlocks, part + kRedBlocks);
   double h = 0.0;
   TB_CUDA(cudaMemcpyAsync(&h, part + kRedBlocks, sizeof(double), cudaMemcpyDeviceToHost, stream));
-  TB_CUDA(cudaFreeAsync(part, stream));
+  sc.put(part);
   TB_CUDA(cudaStreamSynchronize(stream));
   return h;
 }

@@ -290,6 +290,7 @@ int tb_ctx_create(int device, int64_t pool_bytes, tb_ctx* out) {
   auto ctx    = std::make_unique<Ctx>();
   ctx->device = device;
   TB_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
+  ctx->tables = std::make_shared<TableHome>(device, ctx->stream);
   if(pool_bytes <= 0) { // TAMM_GPU_POOL default: 80% of free memory
     size_t fr = 0, tot = 0;
     TB_CUDA(cudaMemGetInfo(&fr, &tot));

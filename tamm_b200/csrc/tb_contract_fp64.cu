@@ -930,8 +930,8 @@ void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, do
   p.A         = A;
   p.B         = B;
   p.C         = C;
-  p.groups    = static_cast<const GroupRec*>(wl.d_group_recs);
-  p.tasks     = static_cast<const TaskRec*>(wl.d_task_recs);
+  p.groups    = reinterpret_cast<const GroupRec*>(wl.d_group_recs);
+  p.tasks     = reinterpret_cast<const TaskRec*>(wl.d_task_recs);
   p.items     = wl.d_items;
   p.err       = wait_error_word();
   p.alpha     = alpha;
@@ -1109,16 +1109,14 @@ static void build_items_fp64(const LabelClasses& lc, const WorkList& wl) {
     tr.reserve(wl.tasks.size());
     for(const auto& g: wl.groups) gr.push_back(group_rec(lc, g));
     for(const auto& t: wl.tasks) tr.push_back(task_rec(lc, t));
-    const size_t gb = sizeof(GroupRec) * gr.size(), tb = sizeof(TaskRec) * tr.size();
-    const size_t ib = sizeof(DevItem) * wl.items_fp64.size();
-    char*        d  = nullptr;
-    TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), gb + tb + ib)); // (the records' sizes are multiples of 16)
-    wl.d_group_recs = d;
-    wl.d_task_recs  = d + gb;
-    wl.d_items      = reinterpret_cast<DevItem*>(d + gb + tb);
-    TB_CUDA(cudaMemcpy(d, gr.data(), gb, cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemcpy(d + gb, tr.data(), tb, cudaMemcpyHostToDevice));
-    TB_CUDA(cudaMemcpy(wl.d_items, wl.items_fp64.data(), ib, cudaMemcpyHostToDevice));
+    GroupRec* dg = nullptr;
+    TaskRec*  dt = nullptr;
+    wl.tables_fp64.add(dg, gr);
+    wl.tables_fp64.add(dt, tr);
+    wl.tables_fp64.add(wl.d_items, wl.items_fp64);
+    wl.tables_fp64.make(wl.home);
+    wl.d_group_recs = reinterpret_cast<char*>(dg);
+    wl.d_task_recs  = reinterpret_cast<char*>(dt);
   }
   wl.ntiles_fp64 = tile;
   wl.split_parts = parts;

@@ -818,23 +818,7 @@ struct I8Layout {
   uint8_t*                d_tslices  = nullptr;
   int*                    d_err     = nullptr;
   int*                    d_ctr     = nullptr; // tile counter of the GEMM's dynamic schedule
-  int                     device    = -1;
-  ~I8Layout() {
-    if(device >= 0) {
-      cudaSetDevice(device);
-      for(SplitSet* x: {&a_staged, &a_general, &b_staged, &b_general}) {
-        cudaFree(x->d_blocks);
-        cudaFree(x->d_cbegin);
-      }
-      cudaFree(d_tasks);
-      cudaFree(d_items);
-      cudaFree(d_meta);
-      cudaFree(d_blockmax);
-      cudaFree(d_tslices);
-      cudaFree(d_err);
-      cudaFree(d_ctr);
-    }
-  }
+  Tables                  tables;
 };
 
 int nt_for(int S) { return S <= 6 ? 80 : 64; }
@@ -1049,27 +1033,20 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
     r0 = r1;
   }
   if(!L->items.empty()) L->kc_per_item /= (double) L->items.size();
-  TB_CUDA(cudaGetDevice(&L->device));
-  auto up = [](auto*& dptr, const auto& vec) {
-    using T = std::remove_reference_t<decltype(vec[0])>;
-    if(vec.empty()) return;
-    TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&dptr), sizeof(T) * vec.size()));
-    TB_CUDA(cudaMemcpy(dptr, vec.data(), sizeof(T) * vec.size(), cudaMemcpyHostToDevice));
-  };
-  for(SplitSet* x: {&L->a_staged, &L->a_general, &L->b_staged, &L->b_general}) {
-    up(x->d_blocks, x->blocks);
-    up(x->d_cbegin, x->cbegin);
-  }
-  up(L->d_tasks, L->tasks);
-  up(L->d_items, L->items);
-  up(L->d_meta, L->meta);
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_blockmax),
-                     sizeof(int32_t) * std::max<size_t>(1, L->a_blocks.size() + L->b_blocks.size())));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_tslices), std::max<size_t>(1, L->tasks.size())));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_err), sizeof(int)));
-  TB_CUDA(cudaMemset(L->d_err, 0, sizeof(int)));
   TB_EXPECTS(L->parts * kArrive < (1ll << 30) && L->items.size() < (1ull << 31), "too many output tiles");
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&L->d_ctr), sizeof(int) * (1 + L->parts * kArrive)));
+  for(SplitSet* x: {&L->a_staged, &L->a_general, &L->b_staged, &L->b_general}) {
+    L->tables.add(x->d_blocks, x->blocks);
+    L->tables.add(x->d_cbegin, x->cbegin);
+  }
+  L->tables.add(L->d_tasks, L->tasks);
+  L->tables.add(L->d_items, L->items);
+  L->tables.add(L->d_meta, L->meta);
+  const std::vector<int> zero(1, 0);
+  L->tables.add(L->d_err, zero);
+  L->tables.room(L->d_blockmax, L->a_blocks.size() + L->b_blocks.size());
+  L->tables.room(L->d_tslices, L->tasks.size());
+  L->tables.room(L->d_ctr, 1 + L->parts * kArrive);
+  L->tables.make(wl.home);
   return L;
 }
 

@@ -4,7 +4,11 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
+#include <memory>
+#include <mutex>
+#include <set>
 #include <stdexcept>
 #include <string>
 #include <tuple>
@@ -86,6 +90,65 @@ struct DevItem {
   int32_t total, nseg;
 };
 
+// Where the small device tables of a context (work lists, layouts, item and block lists)
+// come from.  A plan or scheduler object is often used once, as a user's loop makes a new
+// one per step, and cudaMalloc and cudaFree per table held the host for 25 us and until the
+// device was idle: 93 and 123 of them per three streaming steps of the triples.  Tables
+// come from the device's stream-ordered pool instead, in the order of the context's stream,
+// on which alone they are used, and are filled through a pinned buffer, so that neither
+// making nor dropping one waits for the device.  While the stream is being captured (memory
+// of the pool would become part of the graph) and without a home, cudaMalloc serves.
+class TableHome {
+public:
+  TableHome(int device, cudaStream_t stream): device_(device), stream_(stream) {}
+  ~TableHome();
+  struct Piece {
+    const void* src; // host data (null: left as it is)
+    size_t      bytes, off;
+  };
+  void* make(const std::vector<Piece>& pieces, size_t bytes);
+  void  drop(void* p);
+  void  close(); // the stream is about to go, and is idle
+
+private:
+  bool               capturing() const;
+  std::mutex         mu_;
+  int                device_ = 0;
+  cudaStream_t       stream_ = nullptr;
+  char*              pinned_ = nullptr; // kPinned bytes, the first used_ of them in copies under way
+  size_t             used_   = 0;
+  std::set<void*>    direct_; // tables from cudaMalloc
+  std::vector<void*> late_;   // dropped during a capture
+};
+
+// One device allocation holding several tables.  add() notes a table, make() allocates the
+// block, fills it and sets the tables' pointers; the block goes with the object.
+class Tables {
+public:
+  Tables() = default;
+  Tables(const Tables&) = delete;
+  Tables& operator=(const Tables&) = delete;
+  ~Tables();
+  template<typename T>
+  void add(T*& p, const std::vector<T>& v) {
+    if(!v.empty()) note(reinterpret_cast<void**>(&p), v.data(), sizeof(T) * v.size());
+  }
+  template<typename T>
+  void room(T*& p, size_t n) { // not filled
+    note(reinterpret_cast<void**>(&p), nullptr, sizeof(T) * std::max<size_t>(n, 1));
+  }
+  void make(const std::shared_ptr<TableHome>& home); // on the current device
+
+private:
+  void note(void** p, const void* src, size_t bytes);
+  std::vector<TableHome::Piece> pieces_;
+  std::vector<void**>           ptrs_;
+  size_t                        bytes_ = 0;
+  std::shared_ptr<TableHome>    home_;
+  void*                         base_   = nullptr;
+  int                           device_ = -1;
+};
+
 // Host mirror of a work list plus its device copies.
 struct WorkList {
   std::vector<DevGroup> groups;
@@ -97,12 +160,15 @@ struct WorkList {
   int64_t               ntasks_skipped = 0;
   DevGroup*             d_groups = nullptr;
   DevTask*              d_tasks  = nullptr;
+  std::shared_ptr<TableHome> home; // of the context whose stream runs the list (null: any stream)
+  Tables                tables;
   int                   device   = -1;
   // tile items of the FP64 kernel, built (and uploaded) on its first launch over this
   // work list: contractions that run split-INT8 or BF16x3 never need them
   mutable std::vector<DevItem> items_fp64;
   mutable DevItem*             d_items     = nullptr;
-  mutable void *               d_group_recs = nullptr, *d_task_recs = nullptr; // (d_group_recs: the block of all three)
+  mutable char *               d_group_recs = nullptr, *d_task_recs = nullptr;
+  mutable Tables               tables_fp64;
   mutable bool                 items_built = false;
   mutable int                  items_shape = 64; // tile shape of those items, by its width
   mutable int64_t              ntiles_fp64 = 0;  // output tiles

@@ -107,15 +107,6 @@ LabelClasses classify(const int* cl, int nc, const int* al, int na, const int* b
 
 WorkList::~WorkList() {
   forget_int8_layout(this);
-  if(d_groups || d_tasks || d_group_recs) {
-    int cur = -1;
-    cudaGetDevice(&cur);
-    if(device >= 0) cudaSetDevice(device);
-    cudaFree(d_groups);
-    cudaFree(d_tasks);
-    cudaFree(d_group_recs);
-    if(cur >= 0) cudaSetDevice(cur);
-  }
 }
 
 static void validate_task(const LabelClasses& lc, const DevGroup& g, const DevTask& t) {
@@ -184,14 +175,9 @@ void finalize_worklist(const LabelClasses& lc, WorkList& wl, bool upload) {
   wl.flops = wl.flops_run + wl.flops_skipped;
   if(!upload) return;
   TB_CUDA(cudaGetDevice(&wl.device));
-  auto up = [](auto*& dptr, const auto& vec) {
-    using T = std::remove_reference_t<decltype(vec[0])>;
-    if(vec.empty()) return;
-    TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&dptr), sizeof(T) * vec.size()));
-    TB_CUDA(cudaMemcpy(dptr, vec.data(), sizeof(T) * vec.size(), cudaMemcpyHostToDevice));
-  };
-  up(wl.d_groups, wl.groups);
-  up(wl.d_tasks, wl.tasks);
+  wl.tables.add(wl.d_groups, wl.groups);
+  wl.tables.add(wl.d_tasks, wl.tasks);
+  wl.tables.make(wl.home);
 }
 
 WorkList* single_block_worklist(const LabelClasses& lc, const int64_t* adims, const int64_t* bdims,

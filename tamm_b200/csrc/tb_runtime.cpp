@@ -146,6 +146,115 @@ void check_wait_errors() {
   fail(TB_ERR_TIMEOUT, "FP64 contraction: a device-side wait gave up (code " + std::to_string(h) + ")");
 }
 
+bool TableHome::capturing() const {
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  TB_CUDA(cudaStreamIsCapturing(stream_, &cs));
+  return cs != cudaStreamCaptureStatusNone;
+}
+
+void* TableHome::make(const std::vector<Piece>& pieces, size_t bytes) {
+  constexpr size_t            kPinned = size_t(8) << 20;
+  std::lock_guard<std::mutex> hold(mu_);
+  char*                       p    = nullptr;
+  size_t                      fill = 0; // the filled pieces come first
+  for(const auto& x: pieces)
+    if(x.src) fill = std::max(fill, x.off + x.bytes);
+  if(stream_ == nullptr || capturing()) {
+    TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&p), bytes));
+    direct_.insert(p);
+    for(const auto& x: pieces)
+      if(x.src) TB_CUDA(cudaMemcpy(p + x.off, x.src, x.bytes, cudaMemcpyHostToDevice));
+    return p;
+  }
+  TB_CUDA(cudaMallocFromPoolAsync(reinterpret_cast<void**>(&p), bytes, scratch_pool(), stream_));
+  try {
+    if(fill > kPinned) // (staged by the runtime before each call returns)
+      for(const auto& x: pieces) {
+        if(x.src) TB_CUDA(cudaMemcpyAsync(p + x.off, x.src, x.bytes, cudaMemcpyHostToDevice, stream_));
+      }
+    else if(fill > 0) {
+      if(pinned_ == nullptr)
+        TB_CUDA(cudaHostAlloc(reinterpret_cast<void**>(&pinned_), kPinned, cudaHostAllocDefault));
+      if(used_ + fill > kPinned) { // the copies out of the buffer must be done before it is filled again
+        TB_CUDA(cudaStreamSynchronize(stream_));
+        used_ = 0;
+      }
+      for(const auto& x: pieces)
+        if(x.src) std::memcpy(pinned_ + used_ + x.off, x.src, x.bytes);
+      TB_CUDA(cudaMemcpyAsync(p, pinned_ + used_, fill, cudaMemcpyHostToDevice, stream_));
+      used_ += (fill + 255) & ~size_t(255);
+    }
+  } catch(...) {
+    cudaFreeAsync(p, stream_);
+    throw;
+  }
+  return p;
+}
+
+void TableHome::drop(void* p) {
+  std::lock_guard<std::mutex> hold(mu_);
+  int                         cur = -1;
+  cudaGetDevice(&cur);
+  if(cur != device_) cudaSetDevice(device_);
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  if(direct_.erase(p) > 0 || stream_ == nullptr) cudaFree(p); // (no stream: its work was done before it went)
+  else if(cudaStreamIsCapturing(stream_, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) late_.push_back(p);
+  else {
+    cudaFreeAsync(p, stream_);
+    for(void* q: late_) cudaFreeAsync(q, stream_);
+    late_.clear();
+  }
+  if(cur >= 0 && cur != device_) cudaSetDevice(cur);
+}
+
+void TableHome::close() {
+  std::lock_guard<std::mutex> hold(mu_);
+  for(void* q: late_) cudaFreeAsync(q, stream_);
+  late_.clear();
+  if(pinned_) cudaFreeHost(pinned_);
+  pinned_ = nullptr;
+  stream_ = nullptr;
+}
+
+TableHome::~TableHome() {
+  if(pinned_) cudaFreeHost(pinned_);
+}
+
+void Tables::note(void** p, const void* src, size_t bytes) {
+  pieces_.push_back({src, bytes, bytes_});
+  ptrs_.push_back(p);
+  bytes_ += (bytes + 255) & ~size_t(255);
+}
+
+void Tables::make(const std::shared_ptr<TableHome>& home) {
+  TB_EXPECTS(base_ == nullptr, "tables made twice");
+  const auto   pieces = std::exchange(pieces_, {});
+  const auto   ptrs   = std::exchange(ptrs_, {});
+  const size_t bytes  = std::exchange(bytes_, 0);
+  if(pieces.empty()) return;
+  home_ = home;
+  TB_CUDA(cudaGetDevice(&device_));
+  if(home_) base_ = home_->make(pieces, bytes);
+  else {
+    TB_CUDA(cudaMalloc(&base_, bytes));
+    for(const auto& x: pieces)
+      if(x.src) TB_CUDA(cudaMemcpy(static_cast<char*>(base_) + x.off, x.src, x.bytes, cudaMemcpyHostToDevice));
+  }
+  for(size_t i = 0; i < ptrs.size(); i++) *ptrs[i] = static_cast<char*>(base_) + pieces[i].off;
+}
+
+Tables::~Tables() {
+  if(base_ == nullptr) return;
+  if(home_) home_->drop(base_);
+  else {
+    int cur = -1;
+    cudaGetDevice(&cur);
+    cudaSetDevice(device_);
+    cudaFree(base_);
+    if(cur >= 0) cudaSetDevice(cur);
+  }
+}
+
 void* Scratch::get(int64_t bytes) {
   if(arena) return arena->allocate(bytes);
   void* p = nullptr;
@@ -194,6 +303,7 @@ Ctx::~Ctx() {
         cudaStreamDestroy(x);
       }
     arena.reset();
+    if(tables) tables->close();
     cudaStreamDestroy(stream);
   }
 }
@@ -604,7 +714,8 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
     b_red[i] = find_label(red, b.labels[i]);
   }
 
-  auto wl = std::make_shared<WorkList>();
+  auto wl  = std::make_shared<WorkList>();
+  wl->home = c.t->ctx ? c.t->ctx->tables : nullptr;
   for(int64_t n: c_nt)
     if(n == 0) return wl;
   for(int64_t n: red_nt)
@@ -663,6 +774,7 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
   if(nranks > 1) { // keep the output blocks this rank owns
     const std::vector<int> owner = group_owners(lc, *wl, nranks);
     auto                   mine  = std::make_shared<WorkList>();
+    mine->home                   = wl->home;
     for(size_t gi = 0; gi < wl->groups.size(); gi++) {
       if(owner[gi] != rank) continue;
       mine->flops_skipped += skip_flops[gi];
@@ -686,6 +798,17 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
 }
 
 } // namespace
+
+// A device table of v's elements (one element's room if there are none).
+template<typename T>
+static std::shared_ptr<int64_t> table_of(const std::vector<T>& v, const std::shared_ptr<TableHome>& home) {
+  auto t = std::make_shared<Tables>();
+  T*   d = nullptr;
+  if(v.empty()) t->room(d, 1);
+  else t->add(d, v);
+  t->make(home);
+  return std::shared_ptr<int64_t>(t, reinterpret_cast<int64_t*>(d));
+}
 
 std::shared_ptr<WorkList> mult_worklist(const Op& op, const LabelClasses& lc, bool upload, int rank, int nranks) {
   return build_mult_worklist(op, lc, upload, rank, nranks);
@@ -729,18 +852,7 @@ void Sched::run(Op& op) {
           } while(!it.empty() && next_tuple(it, nt));
         TB_EXPECTS(tri.size() / 3 < (1u << 31), "too many blocks in one map");
         const std::vector<int64_t> segs = seg_list(tri);
-        int64_t*                   d    = nullptr;
-        const int                  dev  = ctx->device;
-        TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), sizeof(int64_t) * std::max<size_t>(segs.size(), 1)));
-        cached = std::shared_ptr<int64_t>(d, [dev](int64_t* q) {
-          int cur = -1;
-          cudaGetDevice(&cur);
-          cudaSetDevice(dev);
-          cudaFree(q);
-          if(cur >= 0) cudaSetDevice(cur);
-        });
-        if(!segs.empty())
-          TB_CUDA(cudaMemcpy(d, segs.data(), sizeof(int64_t) * segs.size(), cudaMemcpyHostToDevice));
+        cached = table_of<int64_t>(segs, ctx->tables);
         count           = (int) (segs.size() / 4);
         seg_total[key]  = segs.empty() ? 0 : segs[segs.size() - 1] + segs[segs.size() - 2];
       }
@@ -789,18 +901,7 @@ void Sched::run(Op& op) {
             tri.push_back((*op.set_blocks)[2 * i + 1]);
           }
           const std::vector<int64_t> segs = seg_list(tri);
-          int64_t*                   d    = nullptr;
-          const int                  dev  = ctx->device;
-          TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), sizeof(int64_t) * std::max<size_t>(segs.size(), 1)));
-          cached = std::shared_ptr<int64_t>(d, [dev](int64_t* p) {
-            int cur = -1;
-            cudaGetDevice(&cur);
-            cudaSetDevice(dev);
-            cudaFree(p);
-            if(cur >= 0) cudaSetDevice(cur);
-          });
-          if(!segs.empty())
-            TB_CUDA(cudaMemcpy(d, segs.data(), sizeof(int64_t) * segs.size(), cudaMemcpyHostToDevice));
+          cached = table_of<int64_t>(segs, ctx->tables);
           map_count[op.fill_key] = (int) (segs.size() / 4);
           seg_total[op.fill_key] = segs.empty() ? 0 : segs[segs.size() - 1] + segs[segs.size() - 2];
         }
@@ -876,18 +977,7 @@ void Sched::run(Op& op) {
         }
         add_units[key] = units;
         TB_EXPECTS(list.size() < (1u << 31), "too many block pairs in one add");
-        BlockAssign* d   = nullptr;
-        const int    dev = ctx->device;
-        TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d), sizeof(BlockAssign) * std::max<size_t>(list.size(), 1)));
-        cached = std::shared_ptr<int64_t>(reinterpret_cast<int64_t*>(d), [dev](int64_t* q) {
-          int cur = -1;
-          cudaGetDevice(&cur);
-          cudaSetDevice(dev);
-          cudaFree(q);
-          if(cur >= 0) cudaSetDevice(cur);
-        });
-        if(!list.empty())
-          TB_CUDA(cudaMemcpy(d, list.data(), sizeof(BlockAssign) * list.size(), cudaMemcpyHostToDevice));
+        cached = table_of<BlockAssign>(list, ctx->tables);
         count = (int) list.size();
       }
       op.add_dev   = cached;
@@ -1030,15 +1120,6 @@ void Sched::prepare_mult(Op& op) {
   op.wl   = wl_cache[sig];
 }
 
-FusedList::~FusedList() {
-  if(!d) return;
-  int cur = -1;
-  cudaGetDevice(&cur);
-  cudaSetDevice(device);
-  cudaFree(d);
-  if(cur >= 0) cudaSetDevice(cur);
-}
-
 // A run of two to four Adds from ops[first] on that share their destination (tensor and
 // labels) and their source tensor, each with the destination's labels in some order - the
 // four terms of P(ab) P(ij), say - goes through one kernel: the destination is read and
@@ -1071,7 +1152,6 @@ void Sched::fuse_adds(size_t first) {
   auto& list = fuse_cache[key];
   if(!list) {
     list         = std::make_shared<FusedList>();
-    list->device = ctx->device;
     list->fits   = true;
     try {
       struct Entry {
@@ -1125,8 +1205,8 @@ void Sched::fuse_adds(size_t first) {
       }
       if(blocks.size() >= (1u << 31)) list->fits = false;
       if(list->fits && !blocks.empty()) {
-        TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&list->d), sizeof(FusedBlock) * blocks.size()));
-        TB_CUDA(cudaMemcpy(list->d, blocks.data(), sizeof(FusedBlock) * blocks.size(), cudaMemcpyHostToDevice));
+        list->tables.add(list->d, blocks);
+        list->tables.make(ctx->tables);
         list->nblocks = (int) blocks.size();
       }
     } catch(const Error&) { // an op that cannot run: reported by the op itself, in its turn
@@ -1281,21 +1361,13 @@ void DenomSpec::build(const Tensor& T, const std::shared_ptr<Ctx>& c, const std:
   ctx     = c;
   nblocks = (int) blocks.size();
   nunits  = (int) units.size();
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_eps), sizeof(double) * std::max<size_t>(eps.size(), 1)));
-  TB_CUDA(cudaMemcpy(d_eps, eps.data(), sizeof(double) * eps.size(), cudaMemcpyHostToDevice));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_blocks), sizeof(DenomBlock) * std::max<size_t>(blocks.size(), 1)));
-  if(!blocks.empty())
-    TB_CUDA(cudaMemcpy(d_blocks, blocks.data(), sizeof(DenomBlock) * blocks.size(), cudaMemcpyHostToDevice));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_units), sizeof(DenomUnit) * std::max<size_t>(units.size(), 1)));
-  if(!units.empty())
-    TB_CUDA(cudaMemcpy(d_units, units.data(), sizeof(DenomUnit) * units.size(), cudaMemcpyHostToDevice));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_part), sizeof(double) * std::max<size_t>(units.size(), 1)));
-}
-
-EnergySpec::~EnergySpec() {
-  if(ctx) cudaSetDevice(ctx->device);
-  if(args.estart) cudaFree(const_cast<int32_t*>(args.estart));
-  if(args.part) cudaFree(args.part);
+  tables.add(d_eps, eps);
+  tables.add(d_blocks, blocks);
+  tables.add(d_units, units);
+  if(eps.empty()) tables.room(d_eps, 1); // (set: the spec is built)
+  if(blocks.empty()) tables.room(d_blocks, 1);
+  tables.room(d_part, units.size());
+  tables.make(c->tables);
 }
 
 // The energy epilogue's device state for a Mult over its work list (see EnergySpec).
@@ -1335,24 +1407,16 @@ static std::shared_ptr<EnergySpec> build_energy(const Op& op, const LabelClasses
     es->npart += Bt * std::max(8 * ((M + 127) / 128) * ((N + 47) / 48), 4 * ((M + 63) / 64) * ((N + 31) / 32));
   }
   int32_t* d_est = nullptr;
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&d_est), sizeof(int32_t) * est.size()));
+  es->tables.add(d_est, est);
+  es->tables.room(es->args.part, (size_t) es->npart);
+  es->tables.make(ctx->tables);
   es->args.estart = d_est;
-  TB_CUDA(cudaMemcpy(d_est, est.data(), sizeof(int32_t) * est.size(), cudaMemcpyHostToDevice));
-  TB_CUDA(cudaMalloc(reinterpret_cast<void**>(&es->args.part), sizeof(double) * std::max<int64_t>(es->npart, 1)));
   std::sort(rest.begin(), rest.end());
   if(!op.denom->d_eps) op.denom->build(C, ctx, &rest); // eps on the device (and the blocks for `rest`)
   es->args.eps = op.denom->d_eps;
   for(int m = 0; m < nc; m++) es->args.sg[m] = op.denom->signs[m];
   if(!rest.empty()) es->rest = op.denom;
   return es;
-}
-
-DenomSpec::~DenomSpec() {
-  if(ctx) cudaSetDevice(ctx->device);
-  if(d_eps) cudaFree(d_eps);
-  if(d_blocks) cudaFree(d_blocks);
-  if(d_part) cudaFree(d_part);
-  if(d_units) cudaFree(d_units);
 }
 
 Graph::~Graph() {

@@ -59,6 +59,7 @@ struct Ctx {
   int                    nslices    = 0;
   int64_t                digit_cache_bytes = 0; // split digits of read-only operands kept, at most
   int64_t                digit_cache_used  = 0;
+  std::shared_ptr<TableHome> tables; // of `stream`
   ~Ctx();
 };
 
@@ -241,10 +242,10 @@ struct Op {
 // Device list of a run of Adds that share one pass (none: nblocks 0 and fits false).
 struct FusedList {
   FusedBlock* d       = nullptr;
-  int         nblocks = 0, staged = 0, device = 0;
+  int         nblocks = 0, staged = 0;
   int64_t     units   = 0;
   bool        fits    = false;
-  ~FusedList();
+  Tables      tables;
 };
 
 // Orbital energies over a root index space (device copy) and per-mode signs of a
@@ -262,7 +263,7 @@ struct DenomSpec {
   void                    build(const Tensor& t, const std::shared_ptr<Ctx>& ctx,
                                 const std::vector<int64_t>* only = nullptr);
   std::shared_ptr<Ctx>    ctx;
-  ~DenomSpec();
+  Tables                  tables;
 };
 
 // Device state of a Mult's energy epilogue, built on its first execution: the
@@ -274,7 +275,7 @@ struct EnergySpec {
   std::shared_ptr<DenomSpec> rest;
   int64_t                    npart = 0;
   std::shared_ptr<Ctx>       ctx;
-  ~EnergySpec();
+  Tables                     tables;
 };
 
 // Choice of the autotuner for one contraction signature and precision request.
