@@ -239,6 +239,7 @@ struct Plan {
   tb_stats     last{};
   Arena*       arena        = nullptr; // scratch source (null: cudaMallocAsync)
   int          tile_n       = 0;       // split-INT8 output tile width (0: default for S)
+  bool         few_uses     = false;   // split-INT8 requested, but FP64 is faster (see few_uses)
   bool         check_errors = true;    // read the device error word after a launch
   // while a CUDA graph is being captured: scratch comes from (and returns to) this
   // pool, which keeps it allocated for the graph's replays

@@ -818,6 +818,38 @@ void run_contract(Plan& plan, const WorkList& wl, double alpha, const double* A,
                   double* C, cudaStream_t stream, Arena* arena); // tb_capi.cpp
 static std::shared_ptr<EnergySpec> build_energy(const Op& op, const LabelClasses& lc, const std::shared_ptr<Ctx>& ctx);
 
+// A contraction asked for in split INT8 that uses each element of its larger operand only a
+// few times: cutting the element into digits (about 10-35 ps each, by layout) then costs
+// more than its FP64 multiply-adds (0.06 ps per use), and INT8 tiles of 80 columns pad a
+// narrow output.  Measured split INT8 / FP64 at S = 6: a tensor times a matrix of N columns
+// 1.7-3.3x at N = 40, 80, 1.3x at 160, 1.1x at 400; square outputs of 100 / 256 / 400 / 784 rows over
+// K = 25600 1.9x / 1.2x / 1.2x / 0.5x.  The line is an output whose rows and columns, M
+// and N, have 1 / M + 1 / N >= 1 / 160; a spin-symmetric operand meets about half of the
+// other side.  Not below 2^20 elements (both sides are a few launches; 8 MB take 15 us to
+// split), nor for a larger operand whose digits are kept, nor at fewer digits than 6, nor where
+// B's last mode is a K label that does not run fastest in the kernels' K order (A's):
+// FP64 reads such a B a sector per element, 62 ms instead of 8.7 at worst.  It follows
+// the tensors alone, not the part of the contraction that a rank or batch runs.
+static bool few_uses(const Op& op, const LabelClasses& lc, const Ctx& c) {
+  if(c.mode != TB_MODE_INT8 || c.nslices != 0 || int8_slices_for(c.err_target) < 6) return false;
+  if(lc.nbatch > 0 || lc.nar > 0 || lc.nbr > 0 || lc.nk == 0) return false;
+  const Tensor &A = *op.a.t, &B = *op.b.t;
+  const Tensor& big = A.nelems >= B.nelems ? A : B;
+  if(big.nelems < (int64_t(1) << 20) || (big.read_only && c.digit_cache_bytes > 0)) return false;
+  if(lc.b_contig == 1 && lc.k_b[lc.nk - 1] != B.nmodes - 1) return false;
+  if(lc.a_contig == 1 && lc.k_a[lc.nk - 1] != A.nmodes - 1) return false;
+  auto outer = [](const Tensor& t, const int8_t* pos, int n) {
+    double x = t.has_spin ? 0.5 : 1.0;
+    for(int j = 0; j < n; j++) {
+      int64_t size = 0;
+      for(int64_t i = 0; i < t.tis[pos[j]]->ntiles(); i++) size += t.tis[pos[j]]->size(i);
+      x *= (double) size;
+    }
+    return std::max(x, 1.0);
+  };
+  return 1.0 / outer(A, lc.m_a, lc.nm) + 1.0 / outer(B, lc.n_b, lc.nn) >= 1.0 / 160;
+}
+
 void Sched::run(Op& op) {
   cudaStream_t st = ctx->stream;
   if(op.kind == Op::Set || op.kind == Op::Add || (op.kind == Op::Mult && !op.energy) || op.kind == Op::Denom ||
@@ -1035,6 +1067,7 @@ void Sched::run(Op& op) {
   op.plan->err_target = ctx->err_target;
   op.plan->nslices    = ctx->nslices;
   op.plan->tile_n     = 0;
+  op.plan->few_uses   = (op.energy || !autotune) && few_uses(op, op.plan->lc, *ctx);
   op.plan->store      = op.store;
   op.plan->energy     = nullptr; // (plans are shared by signature: nothing of an earlier op stays)
   if(op.energy) { // the energy epilogue keeps the context's precision (no autotuning)
