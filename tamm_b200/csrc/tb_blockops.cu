@@ -1145,22 +1145,29 @@ double reduce_dot(const double* x, const double* y, int64_t n, cudaStream_t stre
 //   ENERGY:  part[cta] = sum w^2 / D  (w = t; each CTA sums its units in a fixed
 //            order, k_denom_energy_final sums the CTAs in a fixed order)
 //   update:  t += scale * r / D
+//   DOTS:    update, and for up to two scalar products over the same store, of t (before
+//            the update), r and a third tensor x, part[n * gridDim.x + cta] = the CTA's
+//            share: the energy and the residual norm that end an iteration cost no pass
+//            over t and r of their own.  Bound by memory (t, r, x read, t written).
 constexpr int kDenCols = 1024; // last-mode extents tabulated in shared memory
 constexpr int kDenRows = kDenomUnitRows; // rows of one unit (row parts of D in shared memory)
 
-template<bool ENERGY>
+enum DenomMode { kUpdate, kEnergy, kDots };
+
+template<DenomMode MODE>
 __global__ void __launch_bounds__(kThreads) k_denom(double* __restrict__ t, const double* __restrict__ r, double scale,
                                                     const DenomBlock* __restrict__ blocks,
                                                     const DenomUnit* __restrict__ units, int nunits, int nmodes,
                                                     const double* __restrict__ eps, DenomSigns sg,
-                                                    double* __restrict__ part) {
+                                                    double* __restrict__ part, const DenomDots dots) {
+  constexpr bool ENERGY = MODE == kEnergy;
   __shared__ double drow[kDenRows];
   __shared__ double dcol[kDenCols];
   __shared__ double s_sg[kMaxModes];
   constexpr int     U    = 8; // loads in flight per thread
   const int         tid  = threadIdx.x;
   const int         last = nmodes - 1;
-  double            s    = 0.0;
+  double            s    = 0.0, s1 = 0.0;
   // the signs go to shared memory by static indices, and the blocks' fields are read
   // through a pointer: indexing a copy of either by a runtime mode would put it in
   // local memory (published by the first barrier of the unit loop)
@@ -1168,16 +1175,22 @@ __global__ void __launch_bounds__(kThreads) k_denom(double* __restrict__ t, cons
   for(int m = 0; m < kMaxModes; m++)
     if(tid == m) s_sg[m] = sg.s[m];
   // one element: its value(s) and its denominator
-  auto elem = [&](int64_t i, double v, double w, double D) {
+  auto elem = [&](int64_t i, double v, double w, double x, double D) {
     if constexpr(ENERGY) s += v * v * recip_nr(D);
     else t[i] = v + scale * w * recip_nr(D);
+    if constexpr(MODE == kDots) {
+      auto of = [&](int k) { return k == 0 ? v : k == 1 ? w : x; };
+      s += of(dots.a[0]) * of(dots.b[0]);
+      if(dots.n > 1) s1 += of(dots.a[1]) * of(dots.b[1]);
+    }
   };
-  auto load = [&](int64_t i, double& v, double& w) {
+  auto load = [&](int64_t i, double& v, double& w, double& x) {
     if constexpr(ENERGY) v = __ldg(t + i);
     else {
       v = t[i];
       w = __ldg(r + i);
     }
+    if constexpr(MODE == kDots) x = dots.x ? __ldg(dots.x + i) : 0.0;
   };
   for(int ui = blockIdx.x; ui < nunits; ui += gridDim.x) {
     const DenomUnit                u  = units[ui];
@@ -1210,16 +1223,16 @@ __global__ void __launch_bounds__(kThreads) k_denom(double* __restrict__ t, cons
         const int64_t e0 = base + tid;
         int           k  = 0;
         for(; k + U <= nk; k += U) {
-          double v[U], w[U];
+          double v[U], w[U], x[U];
 #pragma unroll
-          for(int j = 0; j < U; j++) load(e0 + (int64_t) (k + j) * A, v[j], w[j]);
+          for(int j = 0; j < U; j++) load(e0 + (int64_t) (k + j) * A, v[j], w[j], x[j]);
 #pragma unroll
-          for(int j = 0; j < U; j++) elem(e0 + (int64_t) (k + j) * A, v[j], w[j], drow[ro + (k + j) * P] + dc);
+          for(int j = 0; j < U; j++) elem(e0 + (int64_t) (k + j) * A, v[j], w[j], x[j], drow[ro + (k + j) * P] + dc);
         }
         for(; k < nk; k++) {
-          double v, w;
-          load(e0 + (int64_t) k * A, v, w);
-          elem(e0 + (int64_t) k * A, v, w, drow[ro + k * P] + dc);
+          double v, w, x;
+          load(e0 + (int64_t) k * A, v, w, x);
+          elem(e0 + (int64_t) k * A, v, w, x, drow[ro + k * P] + dc);
         }
       }
     }
@@ -1236,43 +1249,49 @@ __global__ void __launch_bounds__(kThreads) k_denom(double* __restrict__ t, cons
         return D;
       };
       for(; e + (U - 1) * kThreads < nel; e += U * kThreads) {
-        double v[U], w[U];
+        double v[U], w[U], x[U];
 #pragma unroll
-        for(int j = 0; j < U; j++) load(base + e + j * kThreads, v[j], w[j]);
+        for(int j = 0; j < U; j++) load(base + e + j * kThreads, v[j], w[j], x[j]);
 #pragma unroll
-        for(int j = 0; j < U; j++) elem(base + e + j * kThreads, v[j], w[j], den());
+        for(int j = 0; j < U; j++) elem(base + e + j * kThreads, v[j], w[j], x[j], den());
       }
       for(; e < nel; e += kThreads) {
-        double v, w;
-        load(base + e, v, w);
-        elem(base + e, v, w, den());
+        double v, w, x;
+        load(base + e, v, w, x);
+        elem(base + e, v, w, x, den());
       }
     }
   }
-  if constexpr(ENERGY) {
+  if constexpr(MODE != kUpdate) {
 #pragma unroll
-    for(int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    __shared__ double ws[kThreads / 32];
-    if((tid & 31) == 0) ws[tid >> 5] = s;
+    for(int o = 16; o > 0; o >>= 1) {
+      s += __shfl_xor_sync(0xffffffffu, s, o);
+      if constexpr(MODE == kDots) s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+    }
+    __shared__ double ws[2][kThreads / 32];
+    if((tid & 31) == 0) {
+      ws[0][tid >> 5] = s;
+      ws[1][tid >> 5] = s1;
+    }
     __syncthreads();
-    if(tid == 0) {
+    if(tid < (MODE == kDots ? dots.n : 1)) {
       double v = 0.0;
-      for(int i = 0; i < kThreads / 32; i++) v += ws[i];
-      part[blockIdx.x] = v;
+      for(int i = 0; i < kThreads / 32; i++) v += ws[tid][i];
+      part[(int64_t) tid * gridDim.x + blockIdx.x] = v;
     }
   }
 }
 
 // Persistent grid of the denominator kernels: as many CTAs as fit on the GPU at once,
 // at most one per unit.
-template<bool ENERGY>
+template<DenomMode MODE>
 int denom_grid(int nunits) {
   static int per_sm[64] = {0};
   int        dev        = 0;
   TB_CUDA(cudaGetDevice(&dev));
   int& k = per_sm[dev < 64 ? dev : 63];
   if(k == 0) {
-    TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_denom<ENERGY>, kThreads, 0));
+    TB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, k_denom<MODE>, kThreads, 0));
     k = std::max(k, 1);
   }
   int nsm = 0;
@@ -1300,10 +1319,10 @@ __global__ void k_set_scalar(double* out, double v) { *out = v; }
 void launch_denom_energy(const double* w, double scale, const DenomBlock* blocks, const DenomUnit* units,
                          int nunits, int nmodes, const double* eps, DenomSigns signs, double* part, double* out,
                          cudaStream_t stream) {
-  const int grid = nunits > 0 ? denom_grid<true>(nunits) : 0;
+  const int grid = nunits > 0 ? denom_grid<kEnergy>(nunits) : 0;
   if(grid > 0)
-    k_denom<true><<<grid, kThreads, 0, stream>>>(const_cast<double*>(w), nullptr, 0.0, blocks, units, nunits, nmodes,
-                                                 eps, signs, part);
+    k_denom<kEnergy><<<grid, kThreads, 0, stream>>>(const_cast<double*>(w), nullptr, 0.0, blocks, units, nunits, nmodes,
+                                                    eps, signs, part, DenomDots{});
   k_denom_energy_final<<<1, 1024, 0, stream>>>(part, grid, scale, out);
   TB_CUDA(cudaGetLastError());
 }
@@ -1334,8 +1353,18 @@ void launch_dot_to(const double* x, const double* y, int64_t n, double scale, in
 void launch_denom(double* t, const double* r, double scale, const DenomBlock* blocks, const DenomUnit* units,
                   int nunits, int nmodes, const double* eps, DenomSigns signs, cudaStream_t stream) {
   if(nunits <= 0) return;
-  k_denom<false><<<denom_grid<false>(nunits), kThreads, 0, stream>>>(t, r, scale, blocks, units, nunits, nmodes, eps,
-                                                                    signs, nullptr);
+  k_denom<kUpdate><<<denom_grid<kUpdate>(nunits), kThreads, 0, stream>>>(t, r, scale, blocks, units, nunits, nmodes,
+                                                                         eps, signs, nullptr, DenomDots{});
+  TB_CUDA(cudaGetLastError());
+}
+
+void launch_denom_dots(double* t, const double* r, double scale, const DenomBlock* blocks, const DenomUnit* units,
+                       int nunits, int nmodes, const double* eps, DenomSigns signs, const DenomDots& dots,
+                       double* part, cudaStream_t stream) {
+  const int grid = denom_grid<kDots>(nunits);
+  k_denom<kDots><<<grid, kThreads, 0, stream>>>(t, r, scale, blocks, units, nunits, nmodes, eps, signs, part, dots);
+  for(int n = 0; n < dots.n; n++)
+    k_dot_final<<<1, 1024, 0, stream>>>(part + (int64_t) n * grid, grid, dots.out[n], dots.scale[n], dots.root[n]);
   TB_CUDA(cudaGetLastError());
 }
 

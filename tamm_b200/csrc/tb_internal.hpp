@@ -392,6 +392,21 @@ struct DenomUnit {
 };
 constexpr int kDenomUnitRows  = 2048;  // at most, so that the row parts fit in shared memory
 constexpr int kDenomUnitElems = 16384; // about, per unit
+// Scalar products taken along with a denominator update over one store: operands a[n] and
+// b[n] are 0 for t as it was before the update, 1 for r, 2 for x; *out[n] = scale[n] * sum
+// (root: of the sum's square root).
+struct DenomDots {
+  const double* x = nullptr;
+  int           n = 0;
+  int8_t        a[2] = {0, 0}, b[2] = {0, 0};
+  int           root[2]  = {0, 0};
+  double        scale[2] = {0, 0};
+  double*       out[2]   = {nullptr, nullptr};
+};
+// (part: 2 nunits doubles of scratch; nunits > 0)
+void launch_denom_dots(double* t, const double* r, double scale, const DenomBlock* blocks, const DenomUnit* units,
+                       int nunits, int nmodes, const double* eps, DenomSigns signs, const DenomDots& dots,
+                       double* part, cudaStream_t stream);
 void launch_denom(double* t, const double* r, double scale, const DenomBlock* blocks, const DenomUnit* units,
                   int nunits, int nmodes, const double* eps, DenomSigns signs, cudaStream_t stream);
 // *out += scale * sum w^2 / D over the blocks (part: nunits doubles of scratch).

@@ -218,6 +218,7 @@ struct Op {
   std::shared_ptr<struct FusedList>      fused;
   FusedOps                               fused_ops{};
   bool                                   fused_done = false;
+  std::vector<Op>                        dots;       // Denom: Dots just before it that run in its kernel
   int                                    fn = 0;     // Map: element function
   std::shared_ptr<int64_t>               map_dev;    // Map: device segment list (seg_list)
   int                                    map_n = 0;  // runs in the list
@@ -256,8 +257,8 @@ struct DenomSpec {
   double*                 d_eps    = nullptr;
   DenomBlock*             d_blocks = nullptr;
   DenomUnit*              d_units  = nullptr; // row work units (kDenomUnitRows / kDenomUnitElems)
-  double*                 d_part   = nullptr; // per-CTA partial sums of the energy reduction
-                                              // (nunits entries: the grid is never larger)
+  double*                 d_part   = nullptr; // per-CTA partial sums of the energy reduction or of
+                                              // two Dots (nunits entries each: the grid is never larger)
   int                     nblocks  = 0, nunits = 0;
   // over the stored blocks of t (only those at the sorted element offsets `only`, if given)
   void                    build(const Tensor& t, const std::shared_ptr<Ctx>& ctx,
@@ -329,6 +330,7 @@ struct Sched {
   void note_zeros(const Op& op, std::map<const Tensor*, std::shared_ptr<std::vector<uint8_t>>>& szero);
   void                                              fuse_assign(Op& set, Op& mult);
   void                                              fuse_adds(size_t first);
+  void                                              fuse_dots(size_t first);
   void                                              tune(Op& op, const std::string& key);
   double*                                           scalars();
   ~Sched();
