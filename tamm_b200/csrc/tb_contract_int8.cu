@@ -839,6 +839,8 @@ void upload_vec(T*& dptr, const std::vector<T>& vec) {
 // launch's other blocks nor on tasks skipped as exact zeros.  A segment takes 0.33 us per
 // step and the last one about 1 us per segment to add them up: at 256 steps both shares of
 // such a contraction are near 50-80 us.
+// BF16x3 cuts between tasks only: its FP32 accumulators hold one task's sum, and cutting
+// that in two would round it differently.
 constexpr int64_t kSplitTiles = 8;
 constexpr int64_t kSplitSteps = 256; // in steps of 32 K elements
 
@@ -851,6 +853,18 @@ void group_segments(const LabelClasses& lc, const WorkList& wl, int32_t group, i
   const int per = kChunkK / kstep; // steps of a 32-element chunk
   for(int t = g.task_begin; t < g.task_end; t++) {
     const int64_t p0 = wl.tasks[t].pos, n = task_chunks(lc, wl.tasks[t]);
+    if(kstep != KC) { // BF16x3: the whole task to the segment of its first chunk
+      int64_t s = p0 * nseg / total;
+      while(total * (s + 1) / nseg <= p0) s++;
+      if(s != seg) {
+        I8Item it{};
+        it.task = t;
+        segs.push_back(it);
+        seg = s;
+      }
+      segs.back().nsteps += L.tasks[t].nkc;
+      continue;
+    }
     for(int64_t c = 0; c < n;) { // the task's chunks, segment by segment
       int64_t s = (p0 + c) * nseg / total;
       while(total * (s + 1) / nseg <= p0 + c) s++;
