@@ -146,9 +146,15 @@ struct I8Params {
 // epilogue warp, at the tile's first segment).
 constexpr int kArrive = 16;
 
+// K steps per pipeline stage: one, or four for the two pieces of BF16x3, whose steps are so
+// short (13 KB, 3 products) that what the producer and the issuer do per stage bounded the
+// kernel: the O=30/V=200 ladder's 1.77 ms with one step per stage became 1.52 with two and
+// 1.30 with four (14 stages of one step: no change).
+__host__ __device__ constexpr int ksteps(int S) { return S == 2 ? 4 : 1; }
+
 template<int S, int NT>
 __host__ __device__ constexpr uint32_t stage_bytes() {
-  return (uint32_t) S * (MT + NT) * KC;
+  return (uint32_t) ksteps(S) * S * (MT + NT) * KC;
 }
 
 constexpr int kTail  = 4608; // barriers, column scales, C offsets and tile records behind the stages
@@ -156,18 +162,20 @@ constexpr int kTailD = 2560; // offset in the tail of the columns' denominator p
 constexpr int kTailT = 3840; // offset in the tail of the queue slots' tile records
 constexpr int kQueue = 4;    // output tiles in flight between producer, MMA issuer and epilogue
 
-// Pipeline depth: as many stages as fit beside the tail, at most 6.
+constexpr int kXStride = 34; // see the transpose buffer below
+constexpr int kXBytes  = 64 * kXStride * 8;
+// Pipeline depth: as many stages as fit beside the tail, at most 6 (BF16x3: beside the tail
+// and the transpose buffer).
 template<int S, int NT>
 __host__ __device__ constexpr int stages() {
-  return (int) ((kMaxSmem - kTail) / stage_bytes<S, NT>()) < 6 ? (int) ((kMaxSmem - kTail) / stage_bytes<S, NT>()) : 6;
+  const int fit = (int) ((kMaxSmem - kTail - (S == 2 ? kXBytes : 0)) / stage_bytes<S, NT>());
+  return fit < 6 ? fit : 6;
 }
 
 // Epilogue transpose buffer behind the tail, where it fits: per epilogue warp XC (8 or
 // 4) columns x 32 rows of doubles, rows kXStride apart (34: the transposed reads of a half
 // warp, 8 columns x 2 rows, fall on 16 distinct bank pairs), 64 columns in all: eight
 // warps of 8 columns, or sixteen of 4.
-constexpr int kXStride = 34;
-constexpr int kXBytes = 64 * kXStride * 8;
 template<int S, int NT>
 __host__ __device__ constexpr bool xpose_fits() {
   return (size_t) stages<S, NT>() * stage_bytes<S, NT>() + kTail + kXBytes <= kMaxSmem;
@@ -191,7 +199,8 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
   static_assert(EW == 8 || (EW == 16 && !EN && !BF), "sixteen epilogue warps: the plain INT8 C update only");
   constexpr int NE = 32 * EW; // epilogue threads
   extern __shared__ __align__(1024) uint8_t smem[];
-  constexpr uint32_t A_BYTES = S * MT * KC, B_BYTES = S * NT * KC, STAGE = A_BYTES + B_BYTES;
+  constexpr int      KS = ksteps(S); // K steps per stage
+  constexpr uint32_t A_BYTES = S * MT * KC, B_BYTES = S * NT * KC, STAGE = KS * (A_BYTES + B_BYTES);
   constexpr int      kStack  = 256 / NT; // B digits per MMA (UMMA N <= 256)
   static_assert(kStack >= 3, "a drain group's three B digits fit one MMA");
   constexpr int      STAGES  = stages<S, NT>();
@@ -309,15 +318,16 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           left -= nkc;
           const uint32_t st = p.tslices[t]; // only the task's leading digits travel
           const uint32_t ab = st * MT * 16, bb = st * NT * 16; // per K half
-          for(int kc = 0; kc < nkc; kc++) {
+          for(int kc = 0; kc < nkc; kc += KS) {
+            const uint32_t n = KS == 1 ? 1 : min(KS, nkc - kc);
             if(!mbar_wait(&empty[stage], phase ^ 1, p.err, 1)) goto done_producer;
-            mbar_arrive_expect_tx(&full[stage], 2 * (ab + bb));
+            mbar_arrive_expect_tx(&full[stage], n * 2 * (ab + bb));
             uint8_t*       sa = smem + stage * STAGE;
             const uint8_t* ka = ga + (int64_t) kc * A_BYTES;
             const uint8_t* kb = gb + (int64_t) kc * B_BYTES;
-            if(st == S) { // both K halves in one copy per operand
-              bulk_g2s(sa, ka, A_BYTES, &full[stage]);
-              bulk_g2s(sa + A_BYTES, kb, B_BYTES, &full[stage]);
+            if(KS > 1 || st == S) { // both K halves (of all the steps) in one copy per operand
+              bulk_g2s(sa, ka, n * A_BYTES, &full[stage]);
+              bulk_g2s(sa + KS * A_BYTES, kb, n * B_BYTES, &full[stage]);
             }
             else
               for(int h = 0; h < 2; h++) {
@@ -361,52 +371,57 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
           const int nkc = min(p.tasks[t].nkc - k0, left);
           const int st  = p.tslices[t];
           left -= nkc;
-          for(int kc = 0; kc < nkc; kc++) {
+          for(int kc = 0; kc < nkc; kc += KS) {
             if(!mbar_wait(&full[stage], phase, p.err, 3)) goto done_mma;
             tc_fence_after();
-            const uint32_t a0 = smem_u32(smem + stage * STAGE), b0 = a0 + A_BYTES;
-            // A digit i times the stacked B digits j0 .. j0 + nd - 1 in one MMA of N =
-            // nd * NT: it adds into the adjacent diagonals i + j0 .. i + j0 + nd - 1
-            if(kc == 0) {
-              // First K step of a task: the previous task's diagonals must have been read
-              // out.  The products go by the epilogue's drain groups of three diagonals
-              // (the same S(S+1)/2 products in as many MMAs), so those into diagonals 0-2
-              // start as soon as the epilogue has read the first group; in each group the
-              // A digit 0 product comes first and overwrites, the others accumulate.
-              int waited = 0;
+            const int steps = KS == 1 ? 1 : min(KS, nkc - kc);
+#pragma unroll 1
+            for(int u = 0; u < steps; u++) {
+              const uint32_t a0 = smem_u32(smem + stage * STAGE) + u * A_BYTES;
+              const uint32_t b0 = smem_u32(smem + stage * STAGE) + KS * A_BYTES + u * B_BYTES;
+              // A digit i times the stacked B digits j0 .. j0 + nd - 1 in one MMA of N =
+              // nd * NT: it adds into the adjacent diagonals i + j0 .. i + j0 + nd - 1
+              if(kc + u == 0) {
+                // First K step of a task: the previous task's diagonals must have been read
+                // out.  The products go by the epilogue's drain groups of three diagonals
+                // (the same S(S+1)/2 products in as many MMAs), so those into diagonals 0-2
+                // start as soon as the epilogue has read the first group; in each group the
+                // A digit 0 product comes first and overwrites, the others accumulate.
+                int waited = 0;
 #pragma unroll
-              for(int g0 = 0; g0 < S; g0 += 3) {
-                const int gl = S - g0 < 3 ? S - g0 : 3;
-                for(; waited < g0 + gl; waited++) {
-                  if(!mbar_wait(&tempty[waited], tphase ^ 1, p.err, 2)) goto done_mma;
-                  tc_fence_after();
-                }
+                for(int g0 = 0; g0 < S; g0 += 3) {
+                  const int gl = S - g0 < 3 ? S - g0 : 3;
+                  for(; waited < g0 + gl; waited++) {
+                    if(!mbar_wait(&tempty[waited], tphase ^ 1, p.err, 2)) goto done_mma;
+                    tc_fence_after();
+                  }
 #pragma unroll
-                for(int i = 0; i < S; i++) {
-                  if(i >= st || i > g0 + gl - 1) break;
-                  const int jlo = g0 - i > 0 ? g0 - i : 0;
-                  const int jhi = min(g0 + gl - 1 - i, st - 1 - i);
-                  if(jlo > jhi) continue;
-                  const int      nd = jhi - jlo + 1; // <= 3 <= kStack
-                  const uint64_t ad = umma_desc_kmajor(a0 + i * MT * 16, S * MT * 16, 128);
-                  const uint64_t bd = umma_desc_kmajor(b0 + jlo * NT * 16, S * NT * 16, 128);
-                  if constexpr(BF) mma_f16(tmem + (i + jlo) * NT, ad, bd, idesc_bf16(MT, nd * NT), i > 0);
-                  else mma_i8(tmem + (i + jlo) * NT, ad, bd, idesc_i8(MT, nd * NT, true, true), i > 0);
+                  for(int i = 0; i < S; i++) {
+                    if(i >= st || i > g0 + gl - 1) break;
+                    const int jlo = g0 - i > 0 ? g0 - i : 0;
+                    const int jhi = min(g0 + gl - 1 - i, st - 1 - i);
+                    if(jlo > jhi) continue;
+                    const int      nd = jhi - jlo + 1; // <= 3 <= kStack
+                    const uint64_t ad = umma_desc_kmajor(a0 + i * MT * 16, S * MT * 16, 128);
+                    const uint64_t bd = umma_desc_kmajor(b0 + jlo * NT * 16, S * NT * 16, 128);
+                    if constexpr(BF) mma_f16(tmem + (i + jlo) * NT, ad, bd, idesc_bf16(MT, nd * NT), i > 0);
+                    else mma_i8(tmem + (i + jlo) * NT, ad, bd, idesc_i8(MT, nd * NT, true, true), i > 0);
+                  }
                 }
               }
-            }
-            else {
+              else {
 #pragma unroll
-              for(int i = 0; i < S; i++) {
-                if(i >= st) break;
-                const uint64_t ad = umma_desc_kmajor(a0 + i * MT * 16, S * MT * 16, 128);
+                for(int i = 0; i < S; i++) {
+                  if(i >= st) break;
+                  const uint64_t ad = umma_desc_kmajor(a0 + i * MT * 16, S * MT * 16, 128);
 #pragma unroll
-                for(int j0 = 0; j0 < S; j0 += kStack) {
-                  if(j0 >= st - i) break;
-                  const int      nd = min(kStack, st - i - j0);
-                  const uint64_t bd = umma_desc_kmajor(b0 + j0 * NT * 16, S * NT * 16, 128);
-                  if constexpr(BF) mma_f16(tmem + (i + j0) * NT, ad, bd, idesc_bf16(MT, nd * NT), true);
-                  else mma_i8(tmem + (i + j0) * NT, ad, bd, idesc_i8(MT, nd * NT, true, true), true);
+                  for(int j0 = 0; j0 < S; j0 += kStack) {
+                    if(j0 >= st - i) break;
+                    const int      nd = min(kStack, st - i - j0);
+                    const uint64_t bd = umma_desc_kmajor(b0 + j0 * NT * 16, S * NT * 16, 128);
+                    if constexpr(BF) mma_f16(tmem + (i + j0) * NT, ad, bd, idesc_bf16(MT, nd * NT), true);
+                    else mma_i8(tmem + (i + j0) * NT, ad, bd, idesc_i8(MT, nd * NT, true, true), true);
+                  }
                 }
               }
             }
