@@ -822,10 +822,11 @@ static std::shared_ptr<EnergySpec> build_energy(const Op& op, const LabelClasses
 // few times: cutting the element into digits (about 10-35 ps each, by layout) then costs
 // more than its FP64 multiply-adds (0.06 ps per use), and INT8 tiles of 80 columns pad a
 // narrow output.  Measured split INT8 / FP64 at S = 6: a tensor times a matrix of N columns
-// 1.7-3.3x at N = 40, 80, 1.3x at 160, 1.1x at 400; square outputs of 100 / 256 / 400 / 784 rows over
-// K = 25600 1.9x / 1.2x / 1.2x / 0.5x.  The line is an output whose rows and columns, M
-// and N, have 1 / M + 1 / N >= 1 / 160; a spin-symmetric operand meets about half of the
-// other side.  Not below 2^20 elements (both sides are a few launches; 8 MB take 15 us to
+// 2.0-2.4x at N = 40, 1.6x at 80, 1.3x at 160; square outputs of 100 / 256 / 784 rows over
+// K = 25600 1.9x / 1.2x / 0.5x; particle ladders, whose integrals have the cheapest split, 1.2x
+// at 72 columns and 0.8x at 98.  The line is an output whose rows and columns, M and N,
+// have 1 / M + 1 / N >= 1 / 80; a spin-symmetric operand meets about half of the other
+// side.  Not below 2^20 elements (both sides are a few launches; 8 MB take 15 us to
 // split), nor for a larger operand whose digits are kept, nor at fewer digits than 6, nor where
 // B's last mode is a K label that does not run fastest in the kernels' K order (A's):
 // FP64 reads such a B a sector per element, 62 ms instead of 8.7 at worst.  It follows
@@ -847,7 +848,7 @@ static bool few_uses(const Op& op, const LabelClasses& lc, const Ctx& c) {
     }
     return std::max(x, 1.0);
   };
-  return 1.0 / outer(A, lc.m_a, lc.nm) + 1.0 / outer(B, lc.n_b, lc.nn) >= 1.0 / 160;
+  return 1.0 / outer(A, lc.m_a, lc.nm) + 1.0 / outer(B, lc.n_b, lc.nn) >= 1.0 / 80;
 }
 
 void Sched::run(Op& op) {

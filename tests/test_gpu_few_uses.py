@@ -15,7 +15,7 @@ def _space(n, t):
 
 @pytest.mark.parametrize("kind,n,target,slices,read_only,fp64", [
     ("dress", 24, 1e-11, 0, False, True), ("dress", 24, 1e-11, 0, True, False), ("dress", 24, 1e-6, 0, False, False),
-    ("dress", 24, 1e-11, 6, False, False), ("dress", 160, 1e-11, 0, False, True), ("dress", 170, 1e-11, 0, False, False),
+    ("dress", 24, 1e-11, 6, False, False), ("dress", 80, 1e-11, 0, False, True), ("dress", 88, 1e-11, 0, False, False),
     ("small", 24, 1e-11, 0, False, False), ("strided", 24, 1e-11, 0, False, False)])
 def test_route(kind, n, target, slices, read_only, fp64):
     ec = tb.ExecutionContext(0, 1 << 31).set_digit_cache(1 << 29)
