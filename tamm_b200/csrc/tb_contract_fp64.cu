@@ -164,10 +164,13 @@ __device__ __forceinline__ double load_now(const double* p) {
   return v;
 }
 
-// Barrier of the producer warps; true if `failed` holds for any of their threads.
+// Barrier of the producer warps; true if `failed` holds for any of their threads.  The
+// barrier counts warps: a warp whose lanes left a wait or a loop one by one has to be
+// together again before it arrives.
 template<int PT>
 __device__ __forceinline__ bool producers_any(bool failed) {
   uint32_t any;
+  __syncwarp();
   asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
                "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
                : "=r"(any)
@@ -478,7 +481,7 @@ __device__ __forceinline__ void consume(const Params& p, Smem<T>& s) {
   uint32_t      phase = 0;
   auto          mrow  = [&](int i) { return wr + i * 16 * T::WM; }; // first row of fragment i
   for(int n = 0;; n++) {
-    if(!mbar_wait(&s.full[stage], phase, p.err, 34) || s.sd[stage].kvalid < 0) return;
+    if(!mbar_wait_warp(&s.full[stage], phase, p.err, 34) || s.sd[stage].kvalid < 0) return;
     const TileGeo<T>& geo   = s.geo[n & 1];
     const int         m_lim = geo.m_lim, n_lim = geo.n_lim;
     const int  nj    = m_lim > wr ? max(0, min(NJ, (n_lim - wn + 7) >> 3)) : 0;
@@ -495,7 +498,7 @@ __device__ __forceinline__ void consume(const Params& p, Smem<T>& s) {
     auto reg = [&](int i, int j, int h) { return ((i * NJ + j) * 4 + h) * CT; }; // slot of an accumulator
     auto has = [&](int i, int j) { return j < nj && (i == 0 || two); };
     for(bool last = false, first = true; !last; first = false) {
-      if(!first && !mbar_wait(&s.full[stage], phase, p.err, 35)) return;
+      if(!first && !mbar_wait_warp(&s.full[stage], phase, p.err, 35)) return;
       const StageInfo d = s.sd[stage];
       last              = d.last != 0;
       if(d.first_step) { // beta chaining of A-only x B-only reduction steps (gemm_wrapper)
@@ -597,13 +600,8 @@ __device__ __forceinline__ void consume(const Params& p, Smem<T>& s) {
 #pragma unroll
           for(int h = 0; h < 4; h++)
             if(has(i, j)) __stcg(w + reg(i, j, h), acc[i][j][h]);
-      __threadfence();
-      __syncwarp();
-      int arrived = 0;
-      if(lane == 0) arrived = atomicAdd(p.cnt + (int64_t) geo.ws * T::NC + warp, 1);
-      write = __shfl_sync(0xffffffffu, arrived, 0) == geo.nparts - 1;
+      write = warp_arrives_last(p.cnt + (int64_t) geo.ws * T::NC + warp, geo.nparts, lane);
       if(write) {
-        __threadfence();
         for(int part = 0; part < geo.nparts; part++) {
           const double* r = w0 + (int64_t) part * (BM * BN);
 #pragma unroll
@@ -691,6 +689,7 @@ __global__ void __launch_bounds__(T::NTHREADS, T::CTAS) k_contract_fp64(const __
     fence_mbarrier_init();
   }
   __syncthreads();
+  __syncwarp(); // (setmaxnreg is warp-wide)
   if(threadIdx.x < T::CT) {
     if constexpr(T::RC > 0) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;\n" ::"n"(T::RC));
     consume<T>(p, s);

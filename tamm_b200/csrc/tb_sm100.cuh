@@ -54,6 +54,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* e
   return false;
 }
 
+// The same for a whole warp: all its lanes agree on the outcome and are together again
+// behind it, as warp-wide instructions (mma.sync, aligned barriers) need them to be.  Every
+// lane waits by itself before, so each has the acquired data.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* err, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, err, code)) != 0;
+}
+
+// Arrival of a warp whose stores to global memory others are to read, at a counter of n
+// arrivals: true for the warp that arrives last, whose lanes may then read what the n - 1
+// others stored (past L1).  The stores of all lanes are ordered before lane 0's fence and
+// arrival by the barrier, the loads of all lanes behind its arrival and fence likewise.
+__device__ __forceinline__ bool warp_arrives_last(int32_t* count, int n, int lane) {
+  __syncwarp();
+  int arrived = 0;
+  if(lane == 0) {
+    __threadfence();
+    asm volatile("atom.acq_rel.gpu.global.add.s32 %0, [%1], 1;\n" : "=r"(arrived) : "l"(count) : "memory");
+    __threadfence();
+  }
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, arrived, 0) == n - 1;
+}
+
 // Global -> shared bulk copy completing on an mbarrier (no cluster multicast).
 __device__ __forceinline__ void bulk_g2s(void* smem_dst, const void* gmem_src, uint32_t bytes,
                                          uint64_t* bar) {
