@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
         // the epilogue threads agree on a timeout, so none is left in a barrier
         const bool got = mbar_wait(&qfull[qslot], qph, p.err, 7);
         uint32_t   anyfail;
+        __syncwarp(); // (the barrier counts warps)
         asm volatile("{\n\t.reg .pred p, q;\n\tsetp.eq.u32 p, %1, 0;\n\t"
                      "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
                      : "=r"(anyfail)
@@ -535,6 +536,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
         // barrier also publishes the scales
         const bool     waited = mbar_wait(tfull, tphase, p.err, 4);
         uint32_t       anyfail;
+        __syncwarp();
         asm volatile("{\n\t.reg .pred p, q;\n\tsetp.eq.u32 p, %1, 0;\n\t"
                      "bar.red.or.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
                      : "=r"(anyfail)
@@ -639,12 +641,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
 #pragma unroll
         for(int x = 0; x < NH; x++)
           if(live && nof[col0 + x] >= 0) __stcg(w + x * NE, racc[x]);
-        __threadfence();
-        __syncwarp();
-        int arrived = 0;
-        if(lane == 0) arrived = atomicAdd(p.ctr + 1 + (int64_t) iws * kArrive + (warp - 2), 1);
-        if(__shfl_sync(0xffffffffu, arrived, 0) != nparts - 1) continue;
-        __threadfence();
+        if(!warp_arrives_last(p.ctr + 1 + (int64_t) iws * kArrive + (warp - 2), nparts, lane)) continue;
 #pragma unroll 1
         for(int y = 0; y < nparts; y++) {
           const double* r = w0 + (int64_t) y * (MT * NT);

@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(32 * (1 + kSplitMaxGroups * kSplitGroup), 1)
     {
       const bool got = mbar_wait(&full[x], round & 1, err, 22);
       uint32_t   anyfail;
+      __syncwarp(); // (the barrier counts warps)
       asm volatile("{\n\t.reg .pred p, q;\n\tsetp.eq.u32 p, %1, 0;\n\t"
                    "bar.red.or.pred q, %2, %3, p;\n\tselp.u32 %0, 1, 0, q;\n\t}\n"
                    : "=r"(anyfail)
