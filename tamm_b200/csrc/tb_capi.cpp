@@ -1398,6 +1398,7 @@ int tb_sched_release(tb_sched s) {
   s->p->wl_cache.clear();
   s->p->fill_cache.clear();
   s->p->fuse_cache.clear();
+  s->p->lambda_tiles.clear();
   TB_API_END
 }
 

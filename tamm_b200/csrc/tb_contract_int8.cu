@@ -140,7 +140,8 @@ struct I8Params {
                            // launch covers completely) instead of C += alpha * result
   int             energy = 0; // set for the EN instantiations: sum (C + alpha * result)^2 / D into en.part
   EnergyArgs      en;
-  double*         ws = nullptr; // sums of split tiles' segments, MT x NT each
+  double*         ws    = nullptr; // sums of split tiles' segments, MT x NT each
+  int             whole = 0;       // there was no memory for them: a split tile's first item runs all of it
 };
 // The tile counter is followed by the arrivals of split tiles, kArrive per segment (one per
 // epilogue warp, at the tile's first segment).
@@ -253,12 +254,18 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
       uint32_t  qph   = 0;
       while(true) { // tiles are handed out longest first, to whichever CTA is free
         if(!mbar_wait(&qempty[qslot], qph ^ 1, p.err, 5)) goto done_producer;
-        const int it = atomicAdd(p.ctr, 1);
+        int it = atomicAdd(p.ctr, 1);
+        if(p.whole)
+          while(it < p.nitems && p.items[it].part > 0) it = atomicAdd(p.ctr, 1);
         qitem[qslot] = it < p.nitems ? it : -1;
         I8Item   item{};
         DevGroup g{};
         if(it < p.nitems) {
           item       = p.items[it];
+          if(p.whole && item.nparts > 1) {
+            item.nparts = 1;
+            item.nsteps = 0x7fffffff;
+          }
           g          = p.groups[item.group];
           TileRec& r = trec[qslot];
           r.c_off      = g.c_off;
@@ -850,16 +857,21 @@ void upload_vec(T*& dptr, const std::vector<T>& vec) {
 // the group's own admitted tasks, run or skipped, so the result depends neither on the
 // launch's other blocks nor on tasks skipped as exact zeros.  A segment takes 0.33 us per
 // step and the last one about 1 us per segment to add them up: at 256 steps both shares of
-// such a contraction are near 50-80 us.
+// such a contraction are near 50-80 us.  Segments keep SMs busy that the contraction's own
+// tiles leave idle, so there are at most kSplitItems over all tiles of the whole contraction
+// (eight per SM of a B200; its workspace at most about 100 MB), and none from half as many
+// tiles on.  That too follows the tensors, not the ranks' or batches' share of them.
 // BF16x3 cuts between tasks only: its FP32 accumulators hold one task's sum, and cutting
 // that in two would round it differently.
-constexpr int64_t kSplitTiles = 8;
+constexpr int64_t kSplitTiles = 8;   // of 128 x 64, whatever the launch's tile width
 constexpr int64_t kSplitSteps = 256; // in steps of 32 K elements
+constexpr int64_t kSplitItems = 1184;
 
 void group_segments(const LabelClasses& lc, const WorkList& wl, int32_t group, int kstep, const I8Layout& L,
                     std::vector<I8Item>& segs) {
   const DevGroup& g     = wl.groups[group];
-  const int64_t   total = wl.group_chunks[group], nseg = (total + kSplitSteps - 1) / kSplitSteps;
+  const int64_t   total = wl.group_chunks[group];
+  const int64_t   nseg  = std::min((total + kSplitSteps - 1) / kSplitSteps, kSplitItems / std::max<int64_t>(wl.out_tiles, 1));
   if(nseg <= 1) return;
   int64_t   seg = -1;
   const int per = kChunkK / kstep; // steps of a 32-element chunk
@@ -1033,7 +1045,7 @@ std::shared_ptr<I8Layout> build_layout(const LabelClasses& lc, const WorkList& w
         for(int64_t nt = 0; nt < gn; nt++, L->ntiles++) {
           I8Item it{order[r].group, (int32_t) mt, (int32_t) nt, (int32_t) L->ntiles, g.task_begin, 0, 0x7fffffff, 0, 1, 0};
           segs.clear();
-          if(gm * gn <= kSplitTiles) group_segments(lc, wl, order[r].group, kstep, *L, segs);
+          if(block_tiles(lc, g.cdims) <= kSplitTiles) group_segments(lc, wl, order[r].group, kstep, *L, segs);
           if(segs.size() <= 1) {
             L->items.push_back(it);
             continue;
@@ -1142,7 +1154,8 @@ void launch_gemm(const I8Layout& L, const WorkList& wl, const LabelClasses& lc, 
     p.energy = 1;
     p.en     = *plan.energy;
   }
-  p.ws = ws;
+  p.ws    = ws;
+  p.whole = L.parts > 0 && ws == nullptr;
   TB_CUDA(cudaMemsetAsync(L.d_ctr, 0, sizeof(int) * (1 + L.parts * kArrive), st));
   const size_t smem = smem_bytes<S, NT>();
   static bool  configured[64][3] = {};
@@ -1299,7 +1312,8 @@ void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* 
   auto* slices = static_cast<uint8_t*>(plan.pinned ? plan.pinned->get(L->slice_bytes) : sc.get(L->slice_bytes));
   auto* exps   = static_cast<int32_t*>(plan.pinned ? plan.pinned->get(ebytes) : sc.get(ebytes));
   const int64_t wbytes = 8 * L->parts * MT * NT; // split tiles' sums
-  auto* ws = wbytes == 0 ? nullptr : static_cast<double*>(plan.pinned ? plan.pinned->get(wbytes) : sc.get(wbytes));
+  Workspace     wsp(plan.arena, plan.pinned, stream);
+  auto*         ws = wbytes == 0 ? nullptr : static_cast<double*>(wsp.get(wbytes));
   cudaEvent_t  evs[3];
   cudaEvent_t* ev = nullptr;
   if(plan.profile) {
@@ -1316,13 +1330,12 @@ void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* 
     case 7: run_s<7>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
     default: run_s<8>(*L, wl, lc, alpha, A, B, C, slices, exps, ws, st, stream, ev); break;
   }
+  wsp.put();
   if(plan.pinned) {
-    if(ws) plan.pinned->put(ws);
     plan.pinned->put(exps);
     plan.pinned->put(slices);
   }
   else {
-    if(ws) sc.put(ws);
     sc.put(exps);
     sc.put(slices);
   }

@@ -154,6 +154,8 @@ struct WorkList {
   std::vector<DevGroup> groups;
   std::vector<DevTask>  tasks;
   std::vector<int32_t>  group_chunks;      // K chunks of each group's admitted tasks, run or skipped
+  int64_t               out_tiles = 0;     // 128 x 64 tiles of the whole contraction's output blocks: of all
+                                           // ranks and batches, whatever part of them this list holds
   double                flops = 0;         // admitted FP64 FLOPs (tasks that run + skipped tasks)
   double                flops_run = 0;     // FP64 FLOPs of the tasks in the list
   double                flops_skipped = 0; // admitted tasks left out: an exactly-zero block of a read-only operand
@@ -272,6 +274,8 @@ void  check_wait_errors();
 void forget_int8_layout(const WorkList* wl);
 // FP64 FLOPs of one task of a group (2 * |C block| * K, times the one-sided steps).
 double task_flops(const LabelClasses& lc, const DevGroup& g, const DevTask& t);
+// 128 x 64 tiles of one output block, over its batch labels.
+int64_t block_tiles(const LabelClasses& lc, const int32_t* cdims);
 // K chunks of one task, over all its one-sided reduction steps.
 int64_t task_chunks(const LabelClasses& lc, const DevTask& t);
 // Largest split-INT8 slice count the error target needs (3..8).

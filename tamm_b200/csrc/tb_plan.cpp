@@ -145,6 +145,14 @@ double task_flops(const LabelClasses& lc, const DevGroup& g, const DevTask& t) {
   return 2.0 * csz * k;
 }
 
+int64_t block_tiles(const LabelClasses& lc, const int32_t* cdims) {
+  int64_t m = 1, n = 1, b = 1;
+  for(int j = 0; j < lc.nm; j++) m *= cdims[lc.m_c[j]];
+  for(int j = 0; j < lc.nn; j++) n *= cdims[lc.n_c[j]];
+  for(int j = 0; j < lc.nbatch; j++) b *= cdims[lc.batch_c[j]];
+  return b * ((m + 127) / 128) * ((n + 63) / 64);
+}
+
 int64_t task_chunks(const LabelClasses& lc, const DevTask& t) {
   int64_t k = 1, steps = 1;
   for(int j = 0; j < lc.nk; j++) k *= t.adims[lc.k_a[j]];
@@ -173,6 +181,8 @@ void finalize_worklist(const LabelClasses& lc, WorkList& wl, bool upload) {
     if(positions) wl.group_chunks[&g - wl.groups.data()] = (int32_t) chunks;
   }
   wl.flops = wl.flops_run + wl.flops_skipped;
+  if(wl.out_tiles == 0)
+    for(const auto& g: wl.groups) wl.out_tiles += block_tiles(lc, g.cdims);
   if(!upload) return;
   TB_CUDA(cudaGetDevice(&wl.device));
   wl.tables.add(wl.d_groups, wl.groups);

@@ -268,6 +268,40 @@ void Scratch::put(void* p) {
   else TB_CUDA(cudaFreeAsync(p, stream));
 }
 
+void* Workspace::get(int64_t bytes) {
+  try {
+    mem_    = pinned_ ? pinned_->get(bytes) : arena_ ? arena_->allocate(bytes) : nullptr;
+    source_ = mem_ == nullptr ? kNone : pinned_ ? kPinned : kArena;
+  } catch(const Error& e) {
+    if(e.code != TB_ERR_NO_MEMORY) throw;
+  }
+  if(mem_) return mem_;
+  const cudaError_t rc = cudaMallocFromPoolAsync(&mem_, (size_t) std::max<int64_t>(bytes, 1), scratch_pool(), stream_);
+  if(rc == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    return mem_ = nullptr;
+  }
+  TB_CUDA(rc);
+  source_ = kPool;
+  return mem_;
+}
+
+void Workspace::put() {
+  void* const p = mem_;
+  mem_          = nullptr;
+  if(p == nullptr) return;
+  if(source_ == kPinned) pinned_->put(p);
+  else if(source_ == kArena) arena_->deallocate(p);
+  else TB_CUDA(cudaFreeAsync(p, stream_));
+}
+
+Workspace::~Workspace() {
+  try {
+    put();
+  } catch(...) {
+  }
+}
+
 void* CapturePool::get(int64_t bytes) {
   bytes = std::max<int64_t>(bytes, 1);
   int best = -1;
@@ -767,14 +801,17 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
     TB_EXPECTS(wl->tasks.size() < (1ull << 31), "too many tasks in one contraction");
     g.task_end = (int32_t) wl->tasks.size();
     wl->groups.push_back(g);
+    wl->out_tiles += block_tiles(lc, g.cdims);
     wl->group_chunks.push_back((int32_t) gchunks);
     skip_flops.push_back(gskip);
     skip_count.push_back(gskipn);
   } while(!cid.empty() && next_tuple(itval, c_nt));
+  if(op.out_tiles > 0) wl->out_tiles = op.out_tiles;
   if(nranks > 1) { // keep the output blocks this rank owns
     const std::vector<int> owner = group_owners(lc, *wl, nranks);
     auto                   mine  = std::make_shared<WorkList>();
     mine->home                   = wl->home;
+    mine->out_tiles              = wl->out_tiles;
     for(size_t gi = 0; gi < wl->groups.size(); gi++) {
       if(owner[gi] != rank) continue;
       mine->flops_skipped += skip_flops[gi];
@@ -1158,7 +1195,8 @@ static std::string zero_key(const std::shared_ptr<const std::vector<uint8_t>>& z
 void Sched::prepare_mult(Op& op) {
   if(op.wl) return;
   const std::string sig = signature(op) + "|owner " + std::to_string(rank) + "/" + std::to_string(nranks) +
-                          "|z " + zero_key(op.za) + " " + zero_key(op.zb);
+                          "|z " + zero_key(op.za) + " " + zero_key(op.zb) +
+                          (op.out_tiles > 0 ? "|t " + std::to_string(op.out_tiles) : "");
   auto              pit = plan_cache.find(sig);
   if(pit == plan_cache.end()) {
     auto plan        = std::make_shared<Plan>();
@@ -1546,6 +1584,29 @@ void Sched::run_lambda_mult(Op& op) {
   }
   const int64_t budget = L.batch_bytes > 0 ? L.batch_bytes
                                            : std::max<int64_t>(64 << 20, (ctx->arena->capacity() - ctx->arena->used()) / 4);
+  // output tiles of the whole contraction: what the batches' kernels decide by it follows
+  // the tensors, not the batches
+  const std::string sig  = signature(op);
+  int64_t&          tiles = lambda_tiles[sig];
+  if(tiles == 0) {
+    const LabelClasses   lc = classify(op.lhs.labels.data(), (int) op.lhs.labels.size(), op.a.labels.data(),
+                                       (int) op.a.labels.size(), op.b.labels.data(), (int) op.b.labels.size());
+    const auto           cm = tile_maps(op.lhs);
+    std::vector<int64_t> nt, it(op.lhs.labels.size(), 0), cid(op.lhs.labels.size());
+    bool                 empty = false;
+    for(const auto& x: op.lhs.ltis) {
+      nt.push_back(x->ntiles());
+      empty |= x->ntiles() == 0;
+    }
+    int32_t dims[kMaxModes];
+    if(!empty) do {
+        for(size_t i = 0; i < cid.size(); i++) cid[i] = cm[i][it[i]];
+        if(!op.lhs.t->is_non_zero(cid.data())) continue;
+        op.lhs.t->block_dims(cid.data(), dims);
+        tiles += block_tiles(lc, dims);
+      } while(!cid.empty() && next_tuple(it, nt));
+  }
+  op.out_tiles = tiles;
   double              flops = 0, flops_run = 0, split_ms = 0, gemm_ms = 0, int8_ops = 0, int8_alg = 0;
   int                 smin = 99, smax = 0;
   const cudaStream_t  st = ctx->stream;

@@ -238,6 +238,7 @@ struct Op {
   // execute (one byte per stored block; null: nothing known): an earlier assignment of
   // the same op list left them without any contribution
   std::shared_ptr<const std::vector<uint8_t>> za, zb;
+  int64_t out_tiles = 0; // output tiles of the whole contraction (of the op, where a batch of it runs)
 };
 
 // Device list of a run of Adds that share one pass (none: nblocks 0 and fits false).
@@ -310,6 +311,7 @@ struct Sched {
   // scheduler that batch builders queue their ops on
   std::map<std::string, std::unique_ptr<tb_tensor_s>> lambda_batches;
   std::unique_ptr<tb_sched_s>                         builder;
+  std::map<std::string, int64_t>                      lambda_tiles; // output tiles of their contractions, by signature
   // work lists of lambda batches run while capturing a graph (their error words are
   // checked by the graph's sync)
   std::vector<std::shared_ptr<WorkList>>              batch_lists;
@@ -351,6 +353,26 @@ struct Graph {
   std::vector<std::shared_ptr<WorkList>> int8_lists;
   std::vector<std::shared_ptr<Plan>>     plans;
   ~Graph();
+};
+
+// Memory that a launch can do without: from the arena (the capture's pool), where that is
+// too short or there is none from the device's stream-ordered pool, else null.
+class Workspace {
+public:
+  Workspace(Arena* arena, CapturePool* pinned, cudaStream_t stream): arena_(arena), pinned_(pinned), stream_(stream) {}
+  Workspace(const Workspace&) = delete;
+  Workspace& operator=(const Workspace&) = delete;
+  ~Workspace();
+  void* get(int64_t bytes);
+  void  put(); // reusable by later work on the stream
+
+private:
+  enum Source { kNone, kArena, kPinned, kPool };
+  Arena*       arena_;
+  CapturePool* pinned_;
+  cudaStream_t stream_;
+  void*        mem_    = nullptr;
+  Source       source_ = kNone;
 };
 
 // scratch memory source for split operands
