@@ -1213,6 +1213,11 @@ void Sched::prepare_mult(Op& op) {
   op.wl   = wl_cache[sig];
 }
 
+// Whether two allocated tensors share no storage (attached ones may).
+static bool apart(const Tensor& x, const Tensor& y) {
+  return x.data && y.data && (x.data + x.nelems <= y.data || y.data + y.nelems <= x.data);
+}
+
 // One or two Dots from ops[first] on with a denominator update t += alpha * r / D right
 // behind them run in the update's kernel if they are over its store: among t, r and at most
 // one more tensor x of as many elements.  Energy, norm and update of 77.8 million amplitudes
@@ -1226,12 +1231,11 @@ void Sched::fuse_dots(size_t first) {
   if(den.kind != Op::Denom || !den.dots.empty() || den.lhs.t == den.a.t) return;
   const Tensor& T = *den.lhs.t;
   const Tensor* x = nullptr;
-  auto          apart = [&](const Tensor& u) { return u.data + u.nelems <= T.data || T.data + T.nelems <= u.data; };
-  if(T.nelems <= 0 || !T.data || !den.a.t->data || den.a.t->nelems != T.nelems || !apart(*den.a.t)) return;
+  if(T.nelems <= 0 || den.a.t->nelems != T.nelems || !apart(T, *den.a.t)) return;
   for(size_t k = 0; k < n; k++)
     for(const Tensor* u: {ops[first + k].a.t, ops[first + k].root ? ops[first + k].a.t : ops[first + k].b.t}) {
       if(u == &T || u == den.a.t) continue;
-      if((x && u != x) || u->is_lambda() || !u->data || u->nelems != T.nelems || !apart(*u)) return;
+      if((x && u != x) || u->is_lambda() || u->nelems != T.nelems || !apart(T, *u)) return;
       x = u;
     }
   try {
@@ -1249,13 +1253,14 @@ void Sched::fuse_dots(size_t first) {
 // labels) and their source tensor, each with the destination's labels in some order - the
 // four terms of P(ab) P(ij), say - goes through one kernel: the destination is read and
 // written once instead of once per op.  Only the first may assign.  Their blocks are those
-// the separate ops would visit (LHSAddPlan: both sides admitted), op by op.
+// the separate ops would visit (LHSAddPlan: both sides admitted), op by op.  Source and
+// destination must not share storage: a later op would have to see what an earlier one wrote.
 void Sched::fuse_adds(size_t first) {
   Op&       head = ops[first];
   const int nd   = head.lhs.t ? head.lhs.t->nmodes : 0;
   auto      fits = [&](const Op& op, bool is_head) {
     if(op.kind != Op::Add || op.fused_done || op.add_blocks || (!is_head && op.is_assign) || op.a.t != head.a.t ||
-       op.a.t == op.lhs.t || op.a.t->is_lambda() || op.a.t->nmodes != nd || !same_target(op.lhs, head.lhs))
+       !apart(*op.a.t, *op.lhs.t) || op.a.t->is_lambda() || op.a.t->nmodes != nd || !same_target(op.lhs, head.lhs))
       return false;
     std::vector<bool> taken(nd, false);
     for(int i = 0; i < nd; i++) {
