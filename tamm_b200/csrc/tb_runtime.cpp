@@ -1222,7 +1222,7 @@ static bool apart(const Tensor& x, const Tensor& y) {
 // behind them run in the update's kernel if they are over its store: among t, r and at most
 // one more tensor x of as many elements.  Energy, norm and update of 77.8 million amplitudes
 // (0.62 GB): four passes over memory instead of six.  Stores attached by the caller that
-// overlap t keep the ops apart.
+// overlap t keep the ops apart, and so does an update that will be refused: its Dots still run.
 void Sched::fuse_dots(size_t first) {
   size_t n = 0;
   while(n < 2 && first + n < ops.size() && ops[first + n].kind == Op::Dot && !ops[first + n].fused_done) n++;
@@ -1231,7 +1231,7 @@ void Sched::fuse_dots(size_t first) {
   if(den.kind != Op::Denom || !den.dots.empty() || den.lhs.t == den.a.t) return;
   const Tensor& T = *den.lhs.t;
   const Tensor* x = nullptr;
-  if(T.nelems <= 0 || den.a.t->nelems != T.nelems || !apart(T, *den.a.t)) return;
+  if(T.read_only || T.nelems <= 0 || den.a.t->nelems != T.nelems || !apart(T, *den.a.t)) return;
   for(size_t k = 0; k < n; k++)
     for(const Tensor* u: {ops[first + k].a.t, ops[first + k].root ? ops[first + k].a.t : ops[first + k].b.t}) {
       if(u == &T || u == den.a.t) continue;

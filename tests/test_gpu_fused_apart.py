@@ -33,3 +33,29 @@ def test_adds_over_one_buffer(labels):
     for t in (R, X):
         t.deallocate()
     ec.close()
+
+
+def test_dots_before_a_refused_update():
+    """The update of a read-only tensor is refused; the dots queued before it have run."""
+    ec = tb.ExecutionContext(0, 1 << 28)
+    S = tb.TiledIndexSpace(tb.IndexSpace(50), [20, 30])
+    t, r = (tb.Tensor([S, S]).allocate(ec) for _ in range(2))
+    rng = np.random.default_rng(4)
+    tv, rv = rng.integers(-8, 8, size=(2, t.nelems)).astype(float)
+    t.write(tv)
+    r.write(rv)
+    t.set_read_only(True)
+    lab = S.labels(2)
+    sch = tb.Scheduler(ec)
+    sch.dot(0, t(*lab), r(*lab))
+    sch.dot(1, r(*lab), r(*lab), 0.5)
+    sch.denom(t(*lab), -1.0, r(*lab), np.ones(50), [1, 1])
+    with pytest.raises(tb.TambError):
+        sch.execute(tb.ExecutionHW.GPU)
+    assert [float(x) for x in sch.scalars(2)] == [tv @ rv, 0.5 * (rv @ rv)]  # sums of small integers: exact
+    t.set_read_only(False)
+    sch.execute(tb.ExecutionHW.GPU)  # the ops are still queued
+    assert np.max(np.abs(t.read() - (tv - rv / 2.0))) <= 1e-14
+    for x in (t, r):
+        x.deallocate()
+    ec.close()
