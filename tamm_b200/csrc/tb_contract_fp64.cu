@@ -18,7 +18,10 @@
 // own leaves its accumulators in a workspace, and the one that arrives last sums them all
 // in order and writes C.  Both give the same bits, and the cuts follow the group's own
 // admitted tasks alone, whether they run or are skipped as exact zeros: a result depends
-// neither on the other blocks of the launch nor on how its work was spread.
+// neither on the other blocks of the launch nor on how its work was spread.  Two exceptions,
+// within the rounding of the sums: one block triple through the block entry is cut into as
+// many parts as its extents and the GPU's SMs ask for, and where not even the closed sums'
+// 82 KB per CTA can be had the segments are not closed.
 //
 // Measured on one B200 (cuBLAS DGEMM: 35.4 TFLOP/s): full 128 x 80 tiles 28 TFLOP/s; the
 // O = 30, V = 180 ladder 7.25 ms (8.19 with one whole 128 x 80 tile per CTA, the gather in
@@ -145,7 +148,7 @@ struct Params {
   EnergyArgs      en;
   int*            err;    // set by a wait that gave up
   int             nitems = 0;
-  double*         ws  = nullptr; // accumulators of split tiles' segments (null: tiles run whole)
+  double*         ws  = nullptr; // accumulators of split tiles' segments (null: each tile's first item runs it whole)
   int32_t*        cnt = nullptr; // arrivals per split tile and warp, from its first part's slot on (zero at launch)
   double*         sum = nullptr; // sums of a whole tile's closed segments, one tile per CTA (null: not closed)
   int32_t*        ctr = nullptr; // items handed out beyond the grid's (zero at launch; null: one per CTA)
@@ -304,7 +307,8 @@ __device__ __forceinline__ void produce(const Params& p, Smem<T>& s) {
       }
       // ---- chunks over (task, reduction step, k0), uniform across the producers ----
       int           t = it.task0, st = 0, k0 = 0, K = 0, ARBR = 0, pos = 0;
-      int           seg = 0, seg_end = it.nseg > 1 ? (int) ((int64_t) it.total / it.nseg) : 0x7fffffff;
+      const int     nseg = it.nparts > 1 ? 1 : it.nseg; // (a part is one segment)
+      int           seg = 0, seg_end = nseg > 1 ? (int) ((int64_t) it.total / nseg) : 0x7fffffff;
       int32_t       kA = 0, kB = 0; // this lane's K element of the chunk: its offsets in the blocks
       const double *a = nullptr, *b = nullptr;
       bool          fresh = true; // a new task begins
@@ -342,7 +346,7 @@ __device__ __forceinline__ void produce(const Params& p, Smem<T>& s) {
         bool close = false;
         while(pos >= seg_end) { // (segments whose tasks are all skipped are passed over)
           seg++;
-          seg_end = seg + 1 < it.nseg ? (int) ((int64_t) it.total * (seg + 1) / it.nseg) : 0x7fffffff;
+          seg_end = seg + 1 < nseg ? (int) ((int64_t) it.total * (seg + 1) / nseg) : 0x7fffffff;
           close   = c > 0;
         }
         const int      kvalid = min(BK, K - k0);
@@ -456,7 +460,12 @@ __device__ __forceinline__ void produce(const Params& p, Smem<T>& s) {
     }
     else n--; // (the geometry slot stays free)
     if(p.ctr == nullptr) break;
-    if(pt == 0) s.next = (int) gridDim.x + atomicAdd(p.ctr, 1);
+    if(pt == 0) {
+      int next = (int) gridDim.x + atomicAdd(p.ctr, 1);
+      if(p.ws == nullptr) // (so that only a CTA's first item can be one to skip: s.next is not written twice between barriers)
+        while(next < p.nitems && p.items[next].part > 0) next = (int) gridDim.x + atomicAdd(p.ctr, 1);
+      s.next = next;
+    }
     if(producers_any<PT>(bad)) goto failed;
     x = s.next;
   }
@@ -739,49 +748,31 @@ constexpr Geo geo_of() {
 }
 Geo geo(int shape) { return shape == 80 ? geo_of<Wide80>() : shape == 64 ? geo_of<Wide64>() : geo_of<Narrow>(); }
 
-// Workspace of a launch: the item counter and the split tiles' arrival counters (cleared
-// here), then a tile of accumulators per part and, for tiles of several segments, per
-// CTA.  Where it cannot be had the tiles run whole, without closing their segments: the
-// same sums in another order.
-struct SplitSpace {
-  Scratch      sc;
-  CapturePool* pinned = nullptr;
-  void*        mem    = nullptr;
-  SplitSpace(Params& p, int64_t parts, int64_t sums, bool counter, const Geo& g, Arena* arena, CapturePool* pin,
-             cudaStream_t stream) {
+// Sets the launch up in workspace: the item counter and the split tiles' arrival counters
+// (cleared here), then a tile of accumulators per part and, for tiles of several segments
+// that run whole, per CTA.  Where the arena has no room for the parts (up to 128 MB) all tiles
+// run whole, closing their segments: the same bits.  Where there is no memory at all for those
+// sums (82 KB per CTA) they run without closing them: the same sums in another order.
+void split_space(Params& p, Workspace& w, int64_t parts, int64_t sums, int64_t grid, bool counter, const Geo& g,
+                 cudaStream_t stream) {
+  const int64_t tile_elems = (int64_t) g.bm * g.bn;
+  for(;;) {
     if(parts == 0 && sums == 0 && !counter) return;
-    sc.arena           = arena;
-    sc.stream          = stream;
-    pinned             = pin;
-    const int64_t tile_elems = (int64_t) g.bm * g.bn, ncnt = 1 + parts * g.warps;
-    const int64_t head = (4 * ncnt + 255) / 256 * 256;
-    const int64_t need = head + 8 * (parts + sums) * tile_elems;
-    try {
-      mem = pinned ? pinned->get(need) : sc.get(need);
-    } catch(const Error& e) {
-      if(e.code != TB_ERR_NO_MEMORY) throw;
-      cudaGetLastError();
+    const int64_t ncnt = 1 + parts * g.warps, head = (4 * ncnt + 255) / 256 * 256;
+    if(void* const mem = w.get(head + 8 * (parts + sums) * tile_elems, parts == 0)) {
+      double* const t = reinterpret_cast<double*>(static_cast<char*>(mem) + head);
+      if(counter) p.ctr = static_cast<int32_t*>(mem);
+      p.cnt = static_cast<int32_t*>(mem) + 1;
+      p.ws  = parts ? t : nullptr;
+      p.sum = sums ? t + parts * tile_elems : nullptr;
+      if(parts || counter) TB_CUDA(cudaMemsetAsync(mem, 0, 4 * ncnt, stream));
       return;
     }
-    if(counter) p.ctr = static_cast<int32_t*>(mem);
-    p.cnt = static_cast<int32_t*>(mem) + 1;
-    p.ws  = reinterpret_cast<double*>(static_cast<char*>(mem) + head);
-    if(sums) p.sum = p.ws + parts * tile_elems;
-    if(parts || counter) TB_CUDA(cudaMemsetAsync(mem, 0, 4 * ncnt, stream));
+    if(parts == 0) return;
+    parts = 0;
+    sums  = grid;
   }
-  void done() { // reusable by later work on the stream
-    if(!mem) return;
-    if(pinned) pinned->put(mem);
-    else sc.put(mem);
-    mem = nullptr;
-  }
-  ~SplitSpace() {
-    try {
-      done();
-    } catch(...) {
-    }
-  }
-};
+}
 
 int64_t ceil_div(int64_t x, int64_t d) { return (x + d - 1) / d; }
 
@@ -945,10 +936,11 @@ void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, do
   const Geo     g      = geo(wl.items_shape);
   const int64_t nitems = (int64_t) wl.items_fp64.size(), slots = (int64_t) sm_count() * g.ctas;
   const int64_t grid   = std::min(nitems, slots);
-  SplitSpace    ws(p, wl.split_parts, wl.multi_segment ? grid : 0, nitems > grid, g, plan.arena, plan.pinned, stream);
+  Workspace     ws(plan.arena, plan.pinned, stream);
+  split_space(p, ws, wl.split_parts, wl.multi_segment ? grid : 0, grid, nitems > grid, g, stream);
   p.nitems = (int) nitems;
   launch_shape(p, wl.items_shape, p.ctr ? grid : nitems, stream);
-  ws.done();
+  ws.put();
   if(plan.energy) launch_energy_final(p.en.part, wl.ntiles_fp64 * g.warps, plan.energy_scale, plan.energy_out, stream);
 }
 
@@ -1001,9 +993,10 @@ void launch_block_fp64(const LabelClasses& lc, const DevGroup& g1, const DevTask
   p.nparts  = (int) nparts;
   p.nchunks = (int) e.chunks;
   TB_EXPECTS(tiles * nparts < (1ll << 31), "work list too large");
-  SplitSpace ws(p, nparts > 1 ? tiles * nparts : 0, 0, false, g, nullptr, nullptr, stream);
+  Workspace ws(nullptr, nullptr, stream);
+  split_space(p, ws, nparts > 1 ? tiles * nparts : 0, 0, 0, false, g, stream);
   launch_shape(p, shape, tiles * nparts, stream);
-  ws.done();
+  ws.put();
 }
 
 // Work items of the FP64 kernel: one per (group, batch index, tile), longest group first
@@ -1089,7 +1082,6 @@ static void build_items_fp64(const LabelClasses& lc, const WorkList& wl) {
           }
           it.nparts = (int32_t) segs.size();
           it.ws     = (int32_t) parts;
-          it.nseg   = 1;
           parts += it.nparts;
           for(const auto& sg: segs) {
             it.task0   = sg.task0;

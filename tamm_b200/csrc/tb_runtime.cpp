@@ -268,14 +268,14 @@ void Scratch::put(void* p) {
   else TB_CUDA(cudaFreeAsync(p, stream));
 }
 
-void* Workspace::get(int64_t bytes) {
+void* Workspace::get(int64_t bytes, bool pool) {
   try {
     mem_    = pinned_ ? pinned_->get(bytes) : arena_ ? arena_->allocate(bytes) : nullptr;
     source_ = mem_ == nullptr ? kNone : pinned_ ? kPinned : kArena;
   } catch(const Error& e) {
     if(e.code != TB_ERR_NO_MEMORY) throw;
   }
-  if(mem_) return mem_;
+  if(mem_ || (!pool && (pinned_ || arena_))) return mem_;
   const cudaError_t rc = cudaMallocFromPoolAsync(&mem_, (size_t) std::max<int64_t>(bytes, 1), scratch_pool(), stream_);
   if(rc == cudaErrorMemoryAllocation) {
     cudaGetLastError();

@@ -356,14 +356,14 @@ struct Graph {
 };
 
 // Memory that a launch can do without: from the arena (the capture's pool), where that is
-// too short or there is none from the device's stream-ordered pool, else null.
+// too short (`pool`) or there is none from the device's stream-ordered pool, else null.
 class Workspace {
 public:
   Workspace(Arena* arena, CapturePool* pinned, cudaStream_t stream): arena_(arena), pinned_(pinned), stream_(stream) {}
   Workspace(const Workspace&) = delete;
   Workspace& operator=(const Workspace&) = delete;
   ~Workspace();
-  void* get(int64_t bytes);
+  void* get(int64_t bytes, bool pool = true);
   void  put(); // reusable by later work on the stream
 
 private:
