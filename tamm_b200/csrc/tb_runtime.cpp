@@ -867,7 +867,8 @@ static std::shared_ptr<EnergySpec> build_energy(const Op& op, const LabelClasses
 // split), nor for a larger operand whose digits are kept, nor at fewer digits than 6, nor where
 // B's last mode is a K label that does not run fastest in the kernels' K order (A's):
 // FP64 reads such a B a sector per element, 62 ms instead of 8.7 at worst.  It follows
-// the tensors alone, not the part of the contraction that a rank or batch runs.
+// the tensors alone (a lambda tensor as a whole), not the part of the contraction that a rank
+// or batch runs.
 static bool few_uses(const Op& op, const LabelClasses& lc, const Ctx& c) {
   if(c.mode != TB_MODE_INT8 || c.nslices != 0 || int8_slices_for(c.err_target) < 6) return false;
   if(lc.nbatch > 0 || lc.nar > 0 || lc.nbr > 0 || lc.nk == 0) return false;
@@ -1126,7 +1127,7 @@ void Sched::run(Op& op) {
   op.plan->err_target = ctx->err_target;
   op.plan->nslices    = ctx->nslices;
   op.plan->tile_n     = 0;
-  op.plan->few_uses   = (op.energy || !autotune) && few_uses(op, op.plan->lc, *ctx);
+  op.plan->few_uses   = (op.energy || !autotune) && (op.few >= 0 ? op.few != 0 : few_uses(op, op.plan->lc, *ctx));
   op.plan->store      = op.store;
   op.plan->energy     = nullptr; // (plans are shared by signature: nothing of an earlier op stays)
   if(op.energy) { // the energy epilogue keeps the context's precision (no autotuning)
@@ -1589,13 +1590,13 @@ void Sched::run_lambda_mult(Op& op) {
   }
   const int64_t budget = L.batch_bytes > 0 ? L.batch_bytes
                                            : std::max<int64_t>(64 << 20, (ctx->arena->capacity() - ctx->arena->used()) / 4);
-  // output tiles of the whole contraction: what the batches' kernels decide by it follows
-  // the tensors, not the batches
-  const std::string sig  = signature(op);
-  int64_t&          tiles = lambda_tiles[sig];
+  // what the batches' kernels are chosen by follows the whole contraction's tensors, not the
+  // batches: whether it uses its operands only a few times, and its output tiles
+  const LabelClasses lc    = classify(op.lhs.labels.data(), (int) op.lhs.labels.size(), op.a.labels.data(),
+                                      (int) op.a.labels.size(), op.b.labels.data(), (int) op.b.labels.size());
+  int64_t&           tiles = lambda_tiles[signature(op)];
+  op.few                   = few_uses(op, lc, *ctx) ? 1 : 0;
   if(tiles == 0) {
-    const LabelClasses   lc = classify(op.lhs.labels.data(), (int) op.lhs.labels.size(), op.a.labels.data(),
-                                       (int) op.a.labels.size(), op.b.labels.data(), (int) op.b.labels.size());
     const auto           cm = tile_maps(op.lhs);
     std::vector<int64_t> nt, it(op.lhs.labels.size(), 0), cid(op.lhs.labels.size());
     bool                 empty = false;

@@ -238,7 +238,9 @@ struct Op {
   // execute (one byte per stored block; null: nothing known): an earlier assignment of
   // the same op list left them without any contribution
   std::shared_ptr<const std::vector<uint8_t>> za, zb;
-  int64_t out_tiles = 0; // output tiles of the whole contraction (of the op, where a batch of it runs)
+  // a batch of a contraction with a lambda operand: what was decided for the whole of it
+  int64_t out_tiles = 0;  // its output tiles
+  int     few       = -1; // see few_uses (-1: not a batch)
 };
 
 // Device list of a run of Adds that share one pass (none: nblocks 0 and fits false).
