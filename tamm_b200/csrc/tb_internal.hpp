@@ -162,7 +162,7 @@ struct WorkList {
   int64_t               ntasks_skipped = 0;
   DevGroup*             d_groups = nullptr;
   DevTask*              d_tasks  = nullptr;
-  std::shared_ptr<TableHome> home; // of the context whose stream runs the list (null: any stream)
+  std::shared_ptr<TableHome> home; // of the scheduler whose stream runs the list (null: any stream)
   Tables                tables;
   int                   device   = -1;
   // tile items of the FP64 kernel, built (and uploaded) on its first launch over this

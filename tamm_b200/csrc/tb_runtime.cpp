@@ -710,8 +710,8 @@ std::vector<int> group_owners(const LabelClasses& lc, const WorkList& wl, int nr
   return owner;
 }
 
-std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& lc, bool upload, int rank,
-                                              int nranks) {
+std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& lc, bool upload, int rank, int nranks,
+                                              const std::shared_ptr<TableHome>& home) {
   const Labeled &c = op.lhs, &a = op.a, &b = op.b;
   auto cm = tile_maps(c), am = tile_maps(a), bm = tile_maps(b);
   // reduction labels: unique rhs labels (A then B) not in the lhs, sorted (multop.hpp:593-601)
@@ -749,7 +749,7 @@ std::shared_ptr<WorkList> build_mult_worklist(const Op& op, const LabelClasses& 
   }
 
   auto wl  = std::make_shared<WorkList>();
-  wl->home = c.t->ctx ? c.t->ctx->tables : nullptr;
+  wl->home = home;
   for(int64_t n: c_nt)
     if(n == 0) return wl;
   for(int64_t n: red_nt)
@@ -848,7 +848,7 @@ static std::shared_ptr<int64_t> table_of(const std::vector<T>& v, const std::sha
 }
 
 std::shared_ptr<WorkList> mult_worklist(const Op& op, const LabelClasses& lc, bool upload, int rank, int nranks) {
-  return build_mult_worklist(op, lc, upload, rank, nranks);
+  return build_mult_worklist(op, lc, upload, rank, nranks, nullptr);
 }
 
 void run_contract(Plan& plan, const WorkList& wl, double alpha, const double* A, const double* B,
@@ -1207,7 +1207,7 @@ void Sched::prepare_mult(Op& op) {
     plan->err_target = ctx->err_target;
     plan->nslices    = ctx->nslices;
     plan_cache[sig]  = plan;
-    wl_cache[sig]    = build_mult_worklist(op, plan->lc, true, rank, nranks);
+    wl_cache[sig]    = build_mult_worklist(op, plan->lc, true, rank, nranks, ctx->tables);
     pit              = plan_cache.find(sig);
   }
   op.plan = pit->second;
