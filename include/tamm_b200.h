@@ -485,8 +485,9 @@ int tb_sched_tune_info(tb_sched s, int64_t index, int* mode, int* tile_n, int* n
  * (building plans, work lists and autotuner choices), then captures the same ops on
  * the context's stream.  tb_graph_launch enqueues one replay; tb_graph_sync waits
  * for it and checks the device error words of its split-INT8 contractions.  The
- * tensors the ops use must stay allocated while the graph exists; the graph keeps
- * the scratch its capture used. */
+ * tensors the ops use, and the scheduler, must stay while the graph exists; the graph
+ * keeps the scratch its capture used and the device tables its kernels read, so the
+ * scheduler may run and release other ops between replays. */
 typedef struct tb_graph_s* tb_graph;
 int tb_sched_graph_create(tb_sched s, tb_graph* out);
 int tb_graph_launch(tb_graph g);

@@ -1337,27 +1337,23 @@ int tb_sched_graph_create(tb_sched s, tb_graph* out) {
   g->ctx        = S.ctx;
   g->pool.arena = S.ctx->arena.get();
   S.pinned      = &g->pool;
+  S.kept        = &g->kept;
   cudaStream_t st = S.ctx->stream;
   TB_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeRelaxed));
   try {
-    for(size_t i = first; i < S.ops.size(); i++) S.run(S.ops[i]);
+    for(size_t i = first; i < S.ops.size(); i++) S.run_kept(S.ops[i]);
   } catch(...) {
     cudaGraph_t dead = nullptr;
     cudaStreamEndCapture(st, &dead);
     if(dead) cudaGraphDestroy(dead);
     S.pinned = nullptr;
+    S.kept   = nullptr;
     throw;
   }
   S.pinned = nullptr;
+  S.kept   = nullptr;
   TB_CUDA(cudaStreamEndCapture(st, &g->graph));
   TB_CUDA(cudaGraphInstantiate(&g->exec, g->graph, 0));
-  for(size_t i = first; i < S.ops.size(); i++)
-    if(S.ops[i].kind == Op::Mult) {
-      if(S.ops[i].wl) g->int8_lists.push_back(S.ops[i].wl);
-      g->plans.push_back(S.ops[i].plan);
-    }
-  for(auto& wl: S.batch_lists) g->int8_lists.push_back(wl); // lambda batches
-  S.batch_lists.clear();
   auto* h = new tb_graph_s();
   h->p    = std::move(g);
   *out    = h;
@@ -1377,7 +1373,7 @@ int tb_graph_sync(tb_graph g) {
   REQUIRE_ARG(g != nullptr);
   TB_CUDA(cudaSetDevice(g->p->ctx->device));
   TB_CUDA(cudaStreamSynchronize(g->p->ctx->stream));
-  for(const auto& wl: g->p->int8_lists) check_int8_errors(*wl, g->p->ctx->stream);
+  for(const auto& x: g->p->kept.layouts) check_int8_errors(x, g->p->ctx->stream);
   check_wait_errors();
   TB_API_END
 }

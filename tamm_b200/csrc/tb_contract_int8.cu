@@ -1397,14 +1397,21 @@ void forget_int8_layout(const WorkList* wl) { g_layouts.erase(wl); }
 
 int int8_slices_for(double err_target) { return slices_for(err_target); }
 
-void check_int8_errors(const WorkList& wl, cudaStream_t stream) {
+void check_int8_errors(const WorkList& wl, cudaStream_t stream) { check_int8_errors(int8_layout(wl), stream); }
+
+std::shared_ptr<void> int8_layout(const WorkList& wl) {
   auto it = g_layouts.find(&wl);
-  if(it == g_layouts.end() || !it->second) return;
-  int h = 0;
-  TB_CUDA(cudaMemcpyAsync(&h, it->second->d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
+  return it == g_layouts.end() ? nullptr : it->second;
+}
+
+void check_int8_errors(const std::shared_ptr<void>& layout, cudaStream_t stream) {
+  if(!layout) return;
+  const I8Layout& L = *static_cast<const I8Layout*>(layout.get());
+  int             h = 0;
+  TB_CUDA(cudaMemcpyAsync(&h, L.d_err, sizeof(int), cudaMemcpyDeviceToHost, stream));
   TB_CUDA(cudaStreamSynchronize(stream));
   if(h != 0) {
-    cudaMemsetAsync(it->second->d_err, 0, sizeof(int), stream);
+    cudaMemsetAsync(L.d_err, 0, sizeof(int), stream);
     fail(TB_ERR_TIMEOUT, "split-INT8 contraction: a device-side wait gave up (code " + std::to_string(h) + ")");
   }
 }

@@ -427,6 +427,10 @@ void launch_block_nonzero(const double* x, const int64_t* pairs, int nblocks, ui
 // Reads and clears the device error word of the split-INT8 launches of a work list;
 // throws TB_ERR_TIMEOUT if a device-side wait gave up.
 void check_int8_errors(const WorkList& wl, cudaStream_t stream);
+// The split layout that the last split launch over a work list used (null: none), to keep
+// its device tables and to check the error word of its launches.
+std::shared_ptr<void> int8_layout(const WorkList& wl);
+void check_int8_errors(const std::shared_ptr<void>& layout, cudaStream_t stream);
 void   launch_fill_random(double* x, int64_t n, uint64_t seed, uint64_t first, int dist, double p0,
                           double p1, cudaStream_t stream);
 

@@ -1645,6 +1645,7 @@ void Sched::run_lambda_mult(Op& op) {
         builder->p->ctx = ctx;
       }
       builder->p->pinned = pinned;
+      builder->p->kept   = kept;
       const int rc = L.lambda_batch(hb.get(), k0, k1, builder.get(), L.lambda_user);
       if(rc != 0) {
         builder->p->ops.clear();
@@ -1653,12 +1654,10 @@ void Sched::run_lambda_mult(Op& op) {
       }
       builder->p->execute(false);
       builder->p->pinned = nullptr;
+      builder->p->kept   = nullptr;
       for(size_t i = builder->p->last_first; i < builder->p->ops.size(); i++) {
         const auto& bo = builder->p->ops[i];
-        if(bo.kind == Op::Mult && bo.wl) {
-          if(pinned) batch_lists.push_back(bo.wl);
-          else if(deferred_checks) pending.push_back(bo.wl);
-        }
+        if(bo.kind == Op::Mult && bo.wl && !pinned && deferred_checks) pending.push_back(bo.wl);
       }
     }
     else {
@@ -1692,11 +1691,8 @@ void Sched::run_lambda_mult(Op& op) {
     for(Labeled* x: {&sub.lhs, &sub.a, &sub.b})
       for(size_t m = 0; m < x->labels.size(); m++)
         if(x->labels[m] == lab0) x->ltis[m] = B.tis[0];
-    run(sub);
-    if(sub.wl) {
-      if(pinned) batch_lists.push_back(sub.wl);
-      else if(deferred_checks) pending.push_back(sub.wl);
-    }
+    run_kept(sub);
+    if(sub.wl && !pinned && deferred_checks) pending.push_back(sub.wl);
     if(sub.plan) {
       const tb_stats& s = sub.plan->last;
       flops += s.flops;
@@ -1725,6 +1721,21 @@ void Sched::run_lambda_mult(Op& op) {
   op.plan->last.slices_max = smax;
   op.plan->last.mode      = ctx->mode;
   op.flops                = flops;
+}
+
+void Kept::add(const Op& op) {
+  for(const std::shared_ptr<void>& x: {std::shared_ptr<void>(op.plan), std::shared_ptr<void>(op.wl),
+                                       std::shared_ptr<void>(op.fused), std::shared_ptr<void>(op.add_dev),
+                                       std::shared_ptr<void>(op.map_dev), std::shared_ptr<void>(op.set_dev),
+                                       std::shared_ptr<void>(op.denom), std::shared_ptr<void>(op.espec)})
+    if(x) objects.push_back(x);
+  if(op.wl)
+    if(auto layout = int8_layout(*op.wl)) layouts.push_back(layout);
+}
+
+void Sched::run_kept(Op& op) {
+  run(op);
+  if(kept) kept->add(op);
 }
 
 // Updates the blocks known to be zero after `op` ran (see Sched::execute).
@@ -1798,7 +1809,7 @@ void Sched::execute(bool profile) {
       fuse_assign(ops[i], ops[i + 1]);
     if(!profile && ops[i].kind == Op::Add) fuse_adds(i); // (a profile times the ops one by one)
     if(!profile && ops[i].kind == Op::Dot) fuse_dots(i);
-    run(ops[i]);
+    run_kept(ops[i]);
     note_zeros(ops[i], szero);
     if(ops[i].kind == Op::Mult && deferred_checks && ops[i].wl) pending.push_back(ops[i].wl);
     if(!pinned) // (a captured graph orders its own ops)

@@ -290,6 +290,14 @@ struct TuneChoice {
   std::vector<int>    modes, tiles;
 };
 
+// Device state that the launches of a capture use and a replay needs again, whatever becomes
+// of the scheduler's caches and ops: tables, plans, work lists; split layouts apart, whose
+// error words the graph's sync checks.
+struct Kept {
+  std::vector<std::shared_ptr<void>> objects, layouts;
+  void                               add(const Op& op);
+};
+
 struct Sched {
   std::shared_ptr<Ctx>                              ctx;
   std::vector<Op>                                   ops;
@@ -314,9 +322,6 @@ struct Sched {
   std::map<std::string, std::unique_ptr<tb_tensor_s>> lambda_batches;
   std::unique_ptr<tb_sched_s>                         builder;
   std::map<std::string, int64_t>                      lambda_tiles; // output tiles of their contractions, by signature
-  // work lists of lambda batches run while capturing a graph (their error words are
-  // checked by the graph's sync)
-  std::vector<std::shared_ptr<WorkList>>              batch_lists;
   // blocks known to be zero by construction at the end of the last execute
   std::map<const Tensor*, std::shared_ptr<std::vector<uint8_t>>> last_zeros;
   void                                                run_lambda_mult(Op& op);
@@ -326,10 +331,12 @@ struct Sched {
   int                                               rank = 0, nranks = 1; // owner-computes share of Mult ops
   std::map<std::string, TuneChoice>                 tune_cache;
   CapturePool*                                      pinned = nullptr; // set while capturing a graph
+  Kept*                                             kept   = nullptr; // likewise
   bool                                              deferred_checks = false; // execute_async
   std::vector<std::shared_ptr<WorkList>>            pending;         // INT8 lists to check at wait()
   void                                              execute(bool profile);
   void                                              run(Op& op);
+  void                                              run_kept(Op& op); // run, and keep what a capture needs
   void                                              prepare_mult(Op& op);
   void note_zeros(const Op& op, std::map<const Tensor*, std::shared_ptr<std::vector<uint8_t>>>& szero);
   void                                              fuse_assign(Op& set, Op& mult);
@@ -346,14 +353,13 @@ void queue_mult_n(Sched& s, const Labeled& lhs, double alpha, const std::vector<
 void mult_n_order(const Labeled& lhs, const std::vector<Labeled>& f, std::vector<int64_t>& pairs, double& cost);
 
 // A captured sequence of scheduler ops: replayed with one graph launch.  Holds the
-// scratch the capture used and the work lists whose error words are checked.
+// scratch and the device state that the capture used.
 struct Graph {
   std::shared_ptr<Ctx>                   ctx;
   cudaGraph_t                            graph = nullptr;
   cudaGraphExec_t                        exec  = nullptr;
   CapturePool                            pool;
-  std::vector<std::shared_ptr<WorkList>> int8_lists;
-  std::vector<std::shared_ptr<Plan>>     plans;
+  Kept                                   kept;
   ~Graph();
 };
 
