@@ -169,7 +169,9 @@ typedef struct tb_stats {
 } tb_stats;
 
 /* C += alpha * sum over tasks of A * B, all groups, one stream-ordered pass.
- * Scratch (INT8 slices) comes from cudaMallocAsync on the stream. */
+ * Scratch (INT8 slices) comes from cudaMallocAsync on the stream.  An FP64 call returns
+ * before its work is done: a device-side wait of it that gave up (TB_ERR_TIMEOUT) is
+ * reported by the next call on the same work list, or by tb_worklist_destroy. */
 int tb_contract(tb_plan plan, tb_worklist wl, double alpha, const double* a, const double* b,
                 double* c, void* stream);
 int tb_plan_stats(tb_plan plan, tb_stats* out);

@@ -129,7 +129,7 @@ struct Tape {
   void run_now() {
     sched.execute(false);
     TB_CUDA(cudaStreamSynchronize(ctx->stream));
-    check_wait_errors();
+    ctx->waits->check();
   }
 
   void forward_contract(const TapeNode& n) {

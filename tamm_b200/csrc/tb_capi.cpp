@@ -123,7 +123,9 @@ int tb_block_multiply(double alpha, const double* a, const int64_t* adims, const
   // A-only / B-only reduction steps are beta-chained on the FP64 tensor-core path.
   const bool fp64 = mode == TB_MODE_FP64 || plan.lc.nar > 0 || plan.lc.nbr > 0;
   finalize_worklist(plan.lc, w, !fp64);
-  if(fp64) launch_block_fp64(plan.lc, w.groups[0], w.tasks[0], alpha, beta, is_assign, a, b, c, st);
+  WaitWord waits;
+  plan.wait_err = waits.device();
+  if(fp64) launch_block_fp64(plan.lc, w.groups[0], w.tasks[0], alpha, beta, is_assign, a, b, c, waits.device(), st);
   else {
     if(is_assign) launch_fill(c, [&] {
         int64_t n = 1;
@@ -133,7 +135,7 @@ int tb_block_multiply(double alpha, const double* a, const int64_t* adims, const
     run_contract(plan, w, alpha, a, b, c, st, nullptr);
   }
   TB_CUDA(cudaStreamSynchronize(st)); // the work list is released on return
-  check_wait_errors();
+  waits.check();
   TB_API_END
 }
 
@@ -250,8 +252,10 @@ int tb_worklist_build(tb_plan plan, int64_t ngroups, const int64_t* group_c_off,
 }
 
 int tb_worklist_destroy(tb_worklist wl) {
-  delete wl;
-  return TB_OK;
+  TB_API_BEGIN
+  std::unique_ptr<tb_worklist_s> own(wl);
+  if(own && own->p->waits) own->p->waits->check();
+  TB_API_END
 }
 
 int tb_worklist_info(tb_worklist wl, int64_t* ntasks, double* flops) {
@@ -267,6 +271,7 @@ int tb_contract(tb_plan plan, tb_worklist wl, double alpha, const double* a, con
   TB_API_BEGIN
   REQUIRE_ARG(plan != nullptr && wl != nullptr);
   REQUIRE_ARG(a != nullptr && b != nullptr && c != nullptr);
+  if(wl->p->waits) wl->p->waits->check(); // of earlier calls
   run_contract(plan->p, *wl->p, alpha, a, b, c, static_cast<cudaStream_t>(stream), nullptr);
   TB_API_END
 }
@@ -291,6 +296,7 @@ int tb_ctx_create(int device, int64_t pool_bytes, tb_ctx* out) {
   ctx->device = device;
   TB_CUDA(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   ctx->tables = std::make_shared<TableHome>(device, ctx->stream);
+  ctx->waits  = std::make_unique<WaitWord>();
   if(pool_bytes <= 0) { // TAMM_GPU_POOL default: 80% of free memory
     size_t fr = 0, tot = 0;
     TB_CUDA(cudaMemGetInfo(&fr, &tot));
@@ -350,7 +356,7 @@ int tb_ctx_synchronize(tb_ctx ctx) {
   TB_CUDA(cudaStreamSynchronize(ctx->p->stream));
   if(ctx->p->h2d) TB_CUDA(cudaStreamSynchronize(ctx->p->h2d));
   if(ctx->p->d2h) TB_CUDA(cudaStreamSynchronize(ctx->p->d2h));
-  check_wait_errors();
+  ctx->p->waits->check();
   TB_API_END
 }
 
@@ -1113,7 +1119,7 @@ int tb_sched_execute(tb_sched s, int hw, int profile) {
   TB_EXPECTS(hw >= 0 && hw <= 2, "hw must be 0 (DEFAULT), 1 (CPU) or 2 (GPU)");
   s->p->execute(profile != 0);
   TB_CUDA(cudaStreamSynchronize(s->p->ctx->stream));
-  check_wait_errors();
+  s->p->ctx->waits->check();
   TB_API_END
 }
 
@@ -1142,7 +1148,7 @@ int tb_sched_wait(tb_sched s) {
   auto pending = std::move(s->p->pending);
   s->p->pending.clear();
   for(const auto& wl: pending) check_int8_errors(*wl, c.stream);
-  check_wait_errors();
+  c.waits->check();
   TB_API_END
 }
 
@@ -1374,7 +1380,7 @@ int tb_graph_sync(tb_graph g) {
   TB_CUDA(cudaSetDevice(g->p->ctx->device));
   TB_CUDA(cudaStreamSynchronize(g->p->ctx->stream));
   for(const auto& x: g->p->kept.layouts) check_int8_errors(x, g->p->ctx->stream);
-  check_wait_errors();
+  g->p->ctx->waits->check();
   TB_API_END
 }
 

@@ -923,7 +923,8 @@ void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, do
   p.groups    = reinterpret_cast<const GroupRec*>(wl.d_group_recs);
   p.tasks     = reinterpret_cast<const TaskRec*>(wl.d_task_recs);
   p.items     = wl.d_items;
-  p.err       = wait_error_word();
+  if(plan.wait_err == nullptr && !wl.waits) wl.waits = std::make_unique<WaitWord>();
+  p.err       = plan.wait_err ? plan.wait_err : wl.waits->device();
   p.alpha     = alpha;
   p.beta      = beta;
   p.is_assign = is_assign;
@@ -950,7 +951,7 @@ void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, do
 // 1073: 78 us per call; 826 us with a work list uploaded per call and 30 whole tiles (the
 // kernel 188 us).
 void launch_block_fp64(const LabelClasses& lc, const DevGroup& g1, const DevTask& t1, double alpha, double beta,
-                       int is_assign, const double* A, const double* B, double* C, cudaStream_t stream) {
+                       int is_assign, const double* A, const double* B, double* C, int* err, cudaStream_t stream) {
   Params p;
   p.lc        = lc;
   p.A         = A;
@@ -959,7 +960,7 @@ void launch_block_fp64(const LabelClasses& lc, const DevGroup& g1, const DevTask
   p.groups    = nullptr;
   p.tasks     = nullptr;
   p.items     = nullptr;
-  p.err       = wait_error_word();
+  p.err       = err;
   p.alpha     = alpha;
   p.beta      = beta;
   p.is_assign = is_assign;

@@ -149,6 +149,23 @@ private:
   int                           device_ = -1;
 };
 
+// Error word of the FP64 contraction's device-side waits, in host memory mapped to the GPU,
+// so that the host reads it without a copy once the launches that may set it have finished.
+// A context has one, and so has each call of the block entry and each work list of a caller's
+// own: a wait that gave up is reported where that work is waited for, and nowhere else.
+class WaitWord {
+public:
+  WaitWord(); // on the current device
+  WaitWord(const WaitWord&) = delete;
+  WaitWord& operator=(const WaitWord&) = delete;
+  ~WaitWord();
+  int* device() const { return device_; }
+  void check(); // throws TB_ERR_TIMEOUT if a wait gave up since the last check, and clears the word
+
+private:
+  int *host_ = nullptr, *device_ = nullptr;
+};
+
 // Host mirror of a work list plus its device copies.
 struct WorkList {
   std::vector<DevGroup> groups;
@@ -162,6 +179,7 @@ struct WorkList {
   int64_t               ntasks_skipped = 0;
   DevGroup*             d_groups = nullptr;
   DevTask*              d_tasks  = nullptr;
+  mutable std::unique_ptr<WaitWord> waits; // of FP64 launches without a context
   std::shared_ptr<TableHome> home; // of the scheduler whose stream runs the list (null: any stream)
   Tables                tables;
   int                   device   = -1;
@@ -243,6 +261,7 @@ struct Plan {
   int          tile_n       = 0;       // split-INT8 output tile width (0: default for S)
   bool         few_uses     = false;   // split-INT8 requested, but FP64 is faster (see few_uses)
   bool         check_errors = true;    // read the device error word after a launch
+  int*         wait_err     = nullptr; // error word of FP64 launches (null: the work list's)
   // while a CUDA graph is being captured: scratch comes from (and returns to) this
   // pool, which keeps it allocated for the graph's replays
   struct CapturePool* pinned = nullptr;
@@ -265,12 +284,6 @@ struct Plan {
   int64_t*      cache_used  = nullptr;
 };
 
-// Error word of the FP64 contraction's device-side waits on the current device, in host
-// memory mapped to the GPU, so that the host reads it without a copy once the launch has
-// finished; check_wait_errors() throws TB_ERR_TIMEOUT if a wait gave up since the last
-// check, and clears it.
-int*  wait_error_word();
-void  check_wait_errors();
 void forget_int8_layout(const WorkList* wl);
 // FP64 FLOPs of one task of a group (2 * |C block| * K, times the one-sided steps).
 double task_flops(const LabelClasses& lc, const DevGroup& g, const DevTask& t);
@@ -287,7 +300,7 @@ void launch_contract_fp64(const Plan& plan, const WorkList& wl, double alpha, do
                           cudaStream_t stream);
 // The same for one block triple, without a work list in device memory.
 void launch_block_fp64(const LabelClasses& lc, const DevGroup& g, const DevTask& t, double alpha, double beta,
-                       int is_assign, const double* A, const double* B, double* C, cudaStream_t stream);
+                       int is_assign, const double* A, const double* B, double* C, int* err, cudaStream_t stream);
 void contract_int8(Plan& plan, const WorkList& wl, double alpha, const double* A,
                    const double* B, double* C, cudaStream_t stream);
 void contract_bf16x3(Plan& plan, const WorkList& wl, double alpha, const double* A,

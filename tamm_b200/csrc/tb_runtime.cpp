@@ -114,36 +114,37 @@ static cudaMemPool_t scratch_pool() {
   return pools[dev];
 }
 
+// Lines of 128 bytes for the wait words, from mapped blocks that stay for the process; a
+// line goes back when its word does.
 namespace {
-int*           g_wait_words = nullptr; // one 128-byte line per device
-std::once_flag g_wait_once;
+std::mutex        g_wait_mu;
+std::vector<int*> g_wait_lines;
 } // namespace
 
-int* wait_error_word() {
-  std::call_once(g_wait_once, [] {
+WaitWord::WaitWord() {
+  constexpr int               kLine = 32, kLines = 64; // ints of a line, lines of a block
+  std::lock_guard<std::mutex> hold(g_wait_mu);
+  if(g_wait_lines.empty()) {
     void* p = nullptr;
-    TB_CUDA(cudaHostAlloc(&p, 64 * 128, cudaHostAllocMapped | cudaHostAllocPortable)); // throws: the flag stays unset
-    std::memset(p, 0, 64 * 128);
-    g_wait_words = static_cast<int*>(p);
-  });
-  int dev = 0;
-  TB_CUDA(cudaGetDevice(&dev));
-  TB_EXPECTS(dev >= 0 && dev < 64, "device index out of range");
+    TB_CUDA(cudaHostAlloc(&p, sizeof(int) * kLine * kLines, cudaHostAllocMapped | cudaHostAllocPortable));
+    for(int i = 0; i < kLines; i++) g_wait_lines.push_back(static_cast<int*>(p) + i * kLine);
+  }
   void* d = nullptr;
-  TB_CUDA(cudaHostGetDevicePointer(&d, g_wait_words + 32 * dev, 0));
-  return static_cast<int*>(d);
+  TB_CUDA(cudaHostGetDevicePointer(&d, g_wait_lines.back(), 0));
+  host_   = g_wait_lines.back();
+  device_ = static_cast<int*>(d);
+  *host_  = 0;
+  g_wait_lines.pop_back();
 }
 
-void check_wait_errors() {
-  if(g_wait_words == nullptr) return;
-  int dev = 0;
-  TB_CUDA(cudaGetDevice(&dev));
-  if(dev < 0 || dev >= 64) return;
-  volatile int* w = g_wait_words + 32 * dev;
-  const int     h = *w;
-  if(h == 0) return;
-  *w = 0;
-  fail(TB_ERR_TIMEOUT, "FP64 contraction: a device-side wait gave up (code " + std::to_string(h) + ")");
+WaitWord::~WaitWord() {
+  std::lock_guard<std::mutex> hold(g_wait_mu);
+  g_wait_lines.push_back(host_);
+}
+
+void WaitWord::check() {
+  const int h = __atomic_exchange_n(host_, 0, __ATOMIC_ACQ_REL);
+  if(h != 0) fail(TB_ERR_TIMEOUT, "FP64 contraction: a device-side wait gave up (code " + std::to_string(h) + ")");
 }
 
 bool TableHome::capturing() const {
@@ -1126,6 +1127,7 @@ void Sched::run(Op& op) {
   op.plan->mode       = ctx->mode;
   op.plan->err_target = ctx->err_target;
   op.plan->nslices    = ctx->nslices;
+  op.plan->wait_err   = ctx->waits->device();
   op.plan->tile_n     = 0;
   op.plan->few_uses   = (op.energy || !autotune) && (op.few >= 0 ? op.few != 0 : few_uses(op, op.plan->lc, *ctx));
   op.plan->store      = op.store;

@@ -60,6 +60,7 @@ struct Ctx {
   int64_t                digit_cache_bytes = 0; // split digits of read-only operands kept, at most
   int64_t                digit_cache_used  = 0;
   std::shared_ptr<TableHome> tables; // of `stream`
+  std::unique_ptr<WaitWord>  waits;  // of its FP64 launches
   ~Ctx();
 };
 
