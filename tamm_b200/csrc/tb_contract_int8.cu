@@ -142,6 +142,7 @@ struct I8Params {
   EnergyArgs      en;
   double*         ws    = nullptr; // sums of split tiles' segments, MT x NT each
   int             whole = 0;       // there was no memory for them: a split tile's first item runs all of it
+  int             ntile = 1;       // without an item list (null: one group, its tiles run whole): tiles per tile row
 };
 // The tile counter is followed by the arrivals of split tiles, kArrive per segment (one per
 // epilogue warp, at the tile's first segment).
@@ -261,7 +262,7 @@ __global__ void __launch_bounds__(64 + 32 * EW, 1) k_contract_i8(const I8Params 
         I8Item   item{};
         DevGroup g{};
         if(it < p.nitems) {
-          item       = p.items[it];
+          item       = p.items ? p.items[it] : I8Item{0, it / p.ntile, it % p.ntile, it, 0, 0, 0x7fffffff, 0, 1, 0};
           if(p.whole && item.nparts > 1) {
             item.nparts = 1;
             item.nsteps = 0x7fffffff;
@@ -1453,7 +1454,9 @@ void*          g_noalloc_base[kNoAllocDevices] = {nullptr};
 std::once_flag g_noalloc_once[kNoAllocDevices];
 
 // Control words and descriptors at fixed offsets of the scratch.
-constexpr int64_t kCtlErr = 0, kCtlCtr = 4, kCtlBlockMax = 8, kCtlSlices = 16, kCtlDesc = 256, kCtlItems = 1280;
+constexpr int64_t kCtlErr = 0, kCtlCtr = 4, kCtlBlockMax = 8, kCtlSlices = 16, kCtlDesc = 256, kCtlEnd = 1280;
+// Counted per output tile in the limit that callers are held to.
+constexpr int64_t kTileBytes = 16;
 
 struct NoAllocDesc {
   SplitBlock a, b;
@@ -1464,13 +1467,13 @@ struct NoAllocDesc {
   int64_t    chunks_off;
 };
 static_assert(kCtlDesc + 2 * sizeof(SplitBlock) + sizeof(DevGroup) + sizeof(I8Task) + sizeof(I8TaskMeta) <=
-                kCtlItems,
-              "descriptor area overflows into the item list");
+                kCtlEnd,
+              "descriptor area");
 
 // Writes the work list and chunk tables of one block triple into the scratch and
 // resets what must start from a known value (error word, block max exponents).
 __global__ void k_noalloc_setup(NoAllocDesc d, unsigned char* base) {
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+  const int tid = threadIdx.x;
   if(tid == 0) {
     *reinterpret_cast<int*>(base + kCtlErr)              = 0;
     *reinterpret_cast<int*>(base + kCtlCtr)              = 0;
@@ -1484,8 +1487,6 @@ __global__ void k_noalloc_setup(NoAllocDesc d, unsigned char* base) {
     *reinterpret_cast<I8TaskMeta*>(reinterpret_cast<I8Task*>(reinterpret_cast<DevGroup*>(sb + 2) + 1) + 1) =
       d.meta;
   }
-  I8Item* items = reinterpret_cast<I8Item*>(base + kCtlItems);
-  for(int i = tid; i < d.mtiles * d.ntiles; i += nth) items[i] = I8Item{0, i / d.ntiles, i % d.ntiles, i, 0, 0, 0x7fffffff, 0, 1, 0};
   if(tid == 0) { // one block per operand: first unit 0, then the unit count
     int32_t* cb = reinterpret_cast<int32_t*>(base + d.chunks_off);
     cb[0] = 0, cb[1] = d.nchunk_a, cb[2] = 0, cb[3] = d.nchunk_b;
@@ -1506,7 +1507,7 @@ void noalloc_launch(const NoAllocDesc& d, unsigned char* base, int64_t exps_off,
   uint8_t*      tsl  = base + kCtlSlices;
   int32_t*      exps = reinterpret_cast<int32_t*>(base + exps_off);
   uint8_t*      sl   = base + slices_off;
-  k_noalloc_setup<<<8, 256, 0, st>>>(d, base);
+  k_noalloc_setup<<<1, 32, 0, st>>>(d, base);
   split_one(S, d.a, sb, cb, A, sl, exps, bmax, st);
   split_one(S, d.b, sb + 1, cb + 2, B, sl, exps, bmax, st);
   k_task_slices<<<1, 32, 0, st>>>(meta, grp, 1, bmax, bmax, S, tsl);
@@ -1517,7 +1518,8 @@ void noalloc_launch(const NoAllocDesc& d, unsigned char* base, int64_t exps_off,
   p.b_exps   = exps;
   p.tasks   = tsk;
   p.groups  = grp;
-  p.items   = reinterpret_cast<const I8Item*>(base + kCtlItems);
+  p.items   = nullptr;
+  p.ntile   = d.ntiles;
   p.nitems  = d.mtiles * d.ntiles;
   p.C       = C;
   p.alpha   = alpha;
@@ -1585,7 +1587,7 @@ extern "C" int tb_block_multiply_int8_noalloc(double alpha, const double* a, con
     const int64_t Mp = rup(M, MT), Np = rup(N, NT), Kp = rup(K, KC);
     const int64_t abytes = S * Mp * Kp, bbytes = S * Np * Kp;
     const int64_t mtiles = Mp / MT, ntiles = Np / NT;
-    const int64_t chunks_off = rup(kCtlItems + (int64_t) sizeof(I8Item) * mtiles * ntiles, 256);
+    const int64_t chunks_off = rup(kCtlEnd + kTileBytes * mtiles * ntiles, 256);
     const int64_t exps_off   = rup(chunks_off + 16, 256);
     const int64_t sl_off     = rup(exps_off + 4 * (Mp + Np), 256);
     const int64_t need       = sl_off + abytes + bbytes;
