@@ -20,14 +20,16 @@ void set_read_only(Tensor& T, bool on);
 // Mode dispatch of one grouped contraction.
 void run_contract(Plan& plan, const WorkList& wl, double alpha, const double* A, const double* B,
                   double* C, cudaStream_t stream, Arena* arena) {
+  // contractions that use the digits too few times to pay for the split run in FP64
+  const int mode     = plan.mode == TB_MODE_INT8 && plan.few_uses ? TB_MODE_FP64 : plan.mode;
   plan.last          = tb_stats{};
   plan.last.flops     = wl.flops;
   plan.last.flops_run = wl.flops_run;
-  plan.last.mode      = plan.mode;
+  plan.last.mode      = mode;
   plan.last.tile_n   = plan.tile_n;
   plan.arena      = arena;
   if(wl.tasks.empty()) return;
-  switch(plan.mode) {
+  switch(mode) {
     case TB_MODE_FP64:
       if(plan.profile) {
         cudaEvent_t e0, e1;

@@ -1289,9 +1289,8 @@ std::shared_ptr<DigitEntry> digit_entry(const Plan& plan, const Tensor* T, int s
 void contract_split(Plan& plan, const WorkList& wl, double alpha, const double* A, const double* B, double* C,
                     cudaStream_t stream, bool bf) {
   const LabelClasses& lc = plan.lc;
-  if(lc.nbatch > 0 || lc.nar > 0 || lc.nbr > 0 || lc.nk == 0 || (!bf && plan.few_uses)) {
-    // Hadamard / one-sided reduction labels and outer products run on the FP64 path, and
-    // so do contractions that use the digits too few times to pay for the split.
+  if(lc.nbatch > 0 || lc.nar > 0 || lc.nbr > 0 || lc.nk == 0) {
+    // Hadamard / one-sided reduction labels and outer products run on the FP64 path.
     launch_contract_fp64(plan, wl, alpha, 1.0, plan.store ? 1 : 0, A, B, C, stream);
     return;
   }

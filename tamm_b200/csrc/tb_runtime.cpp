@@ -1721,7 +1721,7 @@ void Sched::run_lambda_mult(Op& op) {
   op.plan->last.int8_ops_alg = int8_alg;
   op.plan->last.slices_min = smax > 0 ? smin : 0;
   op.plan->last.slices_max = smax;
-  op.plan->last.mode      = ctx->mode;
+  op.plan->last.mode      = op.few > 0 && !autotune ? TB_MODE_FP64 : ctx->mode;
   op.flops                = flops;
 }
 
